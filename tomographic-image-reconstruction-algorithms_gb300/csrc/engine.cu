@@ -82,6 +82,14 @@ struct tomo_ctx {
     bool tile_adj1 = false;
     int tile_warps_fwd = 16, tile_warps_adj = 16;     // tile shape: 16 warps (48 x 48) or 10 (48 x 24)
     int tile_warps_fwd1 = 16, tile_warps_adj1 = 16;   // ... for passes of one group
+    // cluster-resident sweeps (resident.cuh): the shape for passes of P groups and of one group (cpl 0:
+    // off), receivers in row order; slices of the slot, ring and checkpoint buffers are NS floats
+    ResShape res, res1;
+    int64_t NS = 0;
+    int32_t *rchan = nullptr, *rcell = nullptr, *rowstart = nullptr;
+    std::vector<int32_t> h_rowstart;
+    std::vector<ResShape> res_cands;   // every shape that holds a group (tune_resident times them)
+    bool res_tuned = false;
     // learned iteration (allocated on first use)
     float *illum = nullptr, *feat = nullptr, *fsave = nullptr, *dnet = nullptr, *dsave = nullptr;
     unsigned int *illum_max = nullptr, *maxsave = nullptr;
@@ -620,10 +628,10 @@ struct Plan {
 // and residual records.
 double plan_bytes_per_group(const tomo_ctx* c, bool full, int K) {
     const Geometry& g = c->geo;
-    const int64_t N = g.N, nt = g.nt;
+    const int64_t nt = g.nt;
     const int64_t slots = full ? nt : (int64_t)K + 1;
     const int64_t chunks = full ? 0 : (nt - 2 + K - 1) / K;
-    return 4.0 * ((double)(slots + tomo_ctx::ZR + 2 * chunks) * N + (double)nt * g.nch);
+    return 4.0 * ((double)(slots + tomo_ctx::ZR + 2 * chunks) * c->NS + (double)nt * g.nch);
 }
 
 // The plan with the most groups per pass that fits c->plan_budget (or the configured P).
@@ -647,12 +655,31 @@ void set_plan(tomo_ctx* c, const Plan& p) {
     c->nchunk = p.full ? 1 : (nt - 2 + p.K - 1) / p.K;
 }
 
+// Whether the sweeps of this problem stay on chip, with the slice size they need.  The variables that
+// force a strip or tile kernel (tests, profiling) turn them off, as TOMO_RESIDENT=0 does.
+void choose_resident(tomo_ctx* c) {
+    const Geometry& g = c->geo;
+    c->NS = g.N;
+    const char* e = std::getenv("TOMO_RESIDENT");
+    if (g.ref || (e && *e == '0') || std::getenv("TOMO_STRIP_ROWS") || std::getenv("TOMO_TILE") ||
+        std::getenv("TOMO_NO_STRIP"))
+        return;
+    std::vector<int32_t> chan, cell;
+    res_receivers(g.rcv, g.nx, g.ny, chan, cell, c->h_rowstart);
+    c->res_cands = res_shapes(g.nx, g.ny, c->h_rowstart);
+    while (!c->res_cands.empty() && res_held(c->res_cands.back()) < 1) c->res_cands.pop_back();
+    if (c->res_cands.empty()) return;
+    c->res = c->res1 = c->res_cands.back();   // tune_resident picks among them
+    c->NS = res_slice(g.nx, g.ny);
+}
+
 // Chosen memory plan.  ckpt_interval > 0 fixes K; 0 and -1 start from full history when it fits
 // with all groups resident, else K = ceil(sqrt(2 (nt - 2))), the interval of least memory (-1
 // then times the alternatives, tune_plan).
 tomo_status make_plan(tomo_ctx* c) {
     const Geometry& g = c->geo;
     const int64_t N = g.N, nt = g.nt, G = g.G;
+    choose_resident(c);
     size_t free_b = 0, total_b = 0;
     CU(c, cudaMemGetInfo(&free_b, &total_b));
     // fixed buffers (fields, coefficients, accumulators, records)
@@ -681,7 +708,7 @@ tomo_status make_plan(tomo_ctx* c) {
 // records), zeroed.
 tomo_status alloc_plan_buffers(tomo_ctx* c) {
     const Geometry& g = c->geo;
-    const int64_t N = g.N, P = c->P;
+    const int64_t N = c->NS, P = c->P;
     TRY(c->alloc(&c->hist, P * c->S * N, "forward slots"));
     TRY(c->alloc(&c->z, P * tomo_ctx::ZR * N, "adjoint slots"));
     if (!c->full) TRY(c->alloc(&c->ckpt, P * c->nchunk * 2 * N, "checkpoints"));
@@ -711,6 +738,18 @@ tomo_status create_buffers(tomo_ctx* c) {
     TRY(c->alloc(&c->mask, N, "mask"));
     TRY(c->alloc(&c->src, (int64_t)g.src.size(), "source"));
     TRY(c->alloc(&c->rcv, nch, "receivers"));
+    {
+        std::vector<int32_t> chan, cell;
+        res_receivers(g.rcv, g.nx, g.ny, chan, cell, c->h_rowstart);
+        TRY(c->alloc(&c->rchan, (int64_t)chan.size(), "receiver channels in row order"));
+        TRY(c->alloc(&c->rcell, (int64_t)cell.size(), "receiver cells in row order"));
+        TRY(c->alloc(&c->rowstart, g.ny + 1, "receiver rows"));
+        CU(c, cudaMemcpyAsync(c->rchan, chan.data(), sizeof(int32_t) * chan.size(), cudaMemcpyHostToDevice, c->st));
+        CU(c, cudaMemcpyAsync(c->rcell, cell.data(), sizeof(int32_t) * cell.size(), cudaMemcpyHostToDevice, c->st));
+        CU(c, cudaMemcpyAsync(c->rowstart, c->h_rowstart.data(), sizeof(int32_t) * c->h_rowstart.size(),
+                              cudaMemcpyHostToDevice, c->st));
+        TRY(sync_check(c));   // `chan` and `cell` are local
+    }
     if (g.ref) TRY(c->alloc(&c->box, 4 * G, "boxes"));
     else {
         TRY(c->alloc(&c->emit, G * g.gs, "emitters"));
@@ -774,9 +813,109 @@ tomo_status create_buffers(tomo_ctx* c) {
     return TOMO_OK;
 }
 
+// Forward segment of a resident pass: slices k0+1 .. k0+T from the slices at in0, in1 (null: zero).
+ResFwd res_fwd_args(tomo_ctx* c, const ResShape& s, int k0, int T, int g0, int ng) {
+    ResFwd a{};
+    a.coef = c->coef;
+    a.k0 = k0;
+    a.T = T;
+    a.g0 = g0;
+    a.ng = ng;
+    a.cs = s.cs;
+    a.hstride = (int64_t)c->S * c->NS;
+    a.ns = c->NS;
+    a.K = std::max(c->K, 1);
+    a.nchunk = c->nchunk;
+    a.rchan = c->rchan;
+    a.rcell = c->rcell;
+    a.rowstart = c->rowstart;
+    a.w = TileWait{c->err_dev, c->wait_ns, c->test_tx, c->gbar, c->test_gbar};
+    return a;
+}
+
+// Adjoint segment: z(kz0) .. z(kz0-T+1).
+ResAdj res_adj_args(tomo_ctx* c, const ResShape& s, int kz0, int T, int g0, int ng) {
+    ResAdj a{};
+    a.coef = c->coef;
+    a.hist = c->hist;
+    a.hstride = (int64_t)c->S * c->NS;
+    a.ns = c->NS;
+    a.rr = c->rr;
+    a.rrstride = c->recs_per_group();
+    a.rchan = c->rchan;
+    a.rcell = c->rcell;
+    a.rowstart = c->rowstart;
+    a.st = c->z;
+    a.ststride = tomo_ctx::ZR * c->NS;
+    a.corr = c->corr + (int64_t)g0 * c->geo.N;
+    a.cstride = c->geo.N;
+    a.kz0 = kz0;
+    a.T = T;
+    a.ng = ng;
+    a.cs = s.cs;
+    a.w = TileWait{c->err_dev, c->wait_ns, c->test_tx, c->gbar, c->test_gbar};
+    return a;
+}
+
+// A pass by the cluster-resident sweeps: one launch for the forward sweep, one per recomputed chunk
+// and one per chunk of the adjoint sweep.  The forward launches leave L(q) = Laplacian of u(q) in
+// the slots of the chunk being swept.
+int64_t record_resident_pass(tomo_ctx* c, int mode, int g0, int ng) {
+    const Geometry& g = c->geo;
+    const ResShape& s = ng == 1 ? c->res1 : c->res;
+    const int nt = g.nt, K = c->K;
+    const int64_t nch = g.nch, rpg = c->recs_per_group(), cks = (int64_t)c->nchunk * 2 * c->NS;
+    const bool grad = mode == MODE_GRAD, resid = grad || mode == MODE_RESID;
+    int64_t n = 1;
+    ResFwd f = res_fwd_args(c, s, 1, nt - 2, g0, ng);
+    f.gmeas = resid ? c->meas + (int64_t)g0 * rpg : nullptr;
+    f.gout = resid ? c->rr : c->rec + (int64_t)g0 * rpg;
+    if (grad) {
+        f.hist = c->hist;
+        f.qlo = 1 + (c->nchunk - 1) * K;   // the last chunk's (full history: one chunk)
+        if (!c->full) {
+            f.ckpt = c->ckpt;
+            f.ckstride = cks;
+        }
+    } else {   // the last slice, where the caller of a forward solve looks for it
+        f.out = c->hist + c->slot(nt - 1);
+        f.outstride = (int64_t)c->S * g.N;
+    }
+    launch_res_fwd(s, c->dg, f, c->st);
+    if (resid) {
+        launch_resid_parts(c->rr, ng, nt, (int)nch, c->rpart + (int64_t)g0 * nt, c->st);
+        ++n;
+    }
+    if (!grad) return n;
+    for (int ch = c->nchunk - 1; ch >= 0; --ch) {
+        const int qa = 1 + ch * K, qb = std::min(qa + K - 1, nt - 2), T = qb - qa + 1;
+        if (ch < c->nchunk - 1) {
+            const int k = ch > 0 ? res_restart(1, K, ch) : 1;   // newest slice of the chunk's checkpoint
+            ResFwd r = res_fwd_args(c, s, k, qb - k + 1, g0, ng);
+            if (ch > 0) {
+                r.in0 = c->ckpt + (int64_t)ch * 2 * c->NS;
+                r.in1 = r.in0 + c->NS;
+                r.instride = cks;
+            }
+            r.hist = c->hist;
+            r.qlo = qa;
+            launch_res_fwd(s, c->dg, r, c->st);
+            ++n;
+        }
+        ResAdj a = res_adj_args(c, s, qb + 1, T, g0, ng);
+        a.qlo = qa;
+        a.first = ch == c->nchunk - 1;
+        a.last = ch == 0;
+        launch_res_adj(s, c->dg, a, c->st);
+        ++n;
+    }
+    return n;
+}
+
 // Records the launch sequence of one pass (groups g0 .. g0+ng-1) on the stream.
 // Kernel nodes the recorded pass contains (each launch_* call below is one kernel).
 int64_t record_pass(tomo_ctx* c, int mode, int g0, int ng) {
+    if (c->res.cpl && mode != MODE_ILLUM) return record_resident_pass(c, mode, g0, ng);
     int64_t n = 0;
     // multi-step tile kernels: the choice made for passes of one group when the pass has one
     const bool tile_fwd = ng == 1 ? c->tile_fwd1 : c->tile_fwd;
@@ -1006,7 +1145,7 @@ PassLayout pass_layout(const tomo_ctx* c, int mode, int ng) {
     if (L >= nt) return PassLayout{nt, nt - 2, 1, true, false};
     // a pass with full history needs no checkpoints: the checkpoint buffer (P nchunk 2 slices)
     // holds the history when the slot buffer does not (tile kernels need its maps)
-    const bool ck_maps = !(ng == 1 ? c->tile_fwd1 || c->tile_adj1 : c->tile_fwd || c->tile_adj) || c->tmaps_ck.ok;
+    const bool ck_maps = c->res.cpl || !(ng == 1 ? c->tile_fwd1 || c->tile_adj1 : c->tile_fwd || c->tile_adj) || c->tmaps_ck.ok;
     if ((int64_t)c->P * c->nchunk * 2 / ng >= nt && ck_maps) return PassLayout{nt, nt - 2, 1, true, true};
     int nchunk = (int)((nt - 2 + L - 2) / (L - 1));
     int K = (nt - 1 + nchunk - 1) / nchunk;
@@ -1046,11 +1185,101 @@ struct LayoutScope {
     }
 };
 
+// Picks the cluster shapes of the resident sweeps, for passes of P groups and of one, by timing a
+// forward and an adjoint segment of every shape that holds a group on this problem: which of them is
+// fastest depends on how many clusters the GPU holds at once, which only the GPU knows.  All shapes
+// give the same bits.  TOMO_RES_SHAPE="cs,rpw" fixes the choice; TOMO_TUNE_CACHE reuses or records
+// it; TOMO_TUNE_LOG prints each candidate's time.
+tomo_status tune_resident(tomo_ctx* c) {
+    if (c->res_tuned || !c->res.cpl) return TOMO_OK;
+    c->res_tuned = true;
+    const auto& cands = c->res_cands;
+    auto find = [&](int cs, int rpw) -> const ResShape* {
+        for (const ResShape& s : cands)
+            if (s.cs == cs && s.rpw == rpw) return &s;
+        return nullptr;
+    };
+    if (const char* e = std::getenv("TOMO_RES_SHAPE")) {
+        int cs = 0, rpw = 0;
+        if (std::sscanf(e, "%d,%d", &cs, &rpw) == 2)
+            if (const ResShape* s = find(cs, rpw)) {
+                c->res = c->res1 = *s;
+                return TOMO_OK;
+            }
+    }
+    const Geometry& g = c->geo;
+    const char* cache = std::getenv("TOMO_TUNE_CACHE");
+    char key[160];
+    std::snprintf(key, sizeof key, "tomo-res-1 %d %d %d %d %d", g.nx, g.ny, g.nt, c->P, c->S);
+    if (cache && *cache)
+        if (FILE* fp = std::fopen(cache, "r")) {
+            char line[512];
+            bool hit = false;
+            while (!hit && std::fgets(line, sizeof line, fp)) {
+                int v[4];
+                const size_t n = std::strlen(key);
+                if (std::strncmp(line, key, n) != 0 || line[n] != ' ' ||
+                    std::sscanf(line + n, "%d %d %d %d", &v[0], &v[1], &v[2], &v[3]) != 4)
+                    continue;
+                const ResShape *p = find(v[0], v[1]), *o = find(v[2], v[3]);
+                if (p && o) {
+                    c->res = *p;
+                    c->res1 = *o;
+                    hit = true;
+                }
+            }
+            std::fclose(fp);
+            if (hit) return TOMO_OK;
+        }
+    const bool tlog = std::getenv("TOMO_TUNE_LOG") != nullptr;
+    const int T = std::min(std::min(c->K, g.nt - 2), 48);
+    for (int which = 0; which < (c->P > 1 ? 2 : 1); ++which) {
+        const int ng = which == 0 ? 1 : c->P;
+        float best = 1e30f;
+        for (const ResShape& s : cands) {
+            if (res_held(s) < 1) continue;
+            float ms = 1e30f;
+            for (int pass = 0; pass < 3; ++pass) {   // the first warms up
+                ResFwd f = res_fwd_args(c, s, 1, T, 0, ng);
+                f.hist = c->hist;
+                f.qlo = 1;
+                ResAdj a = res_adj_args(c, s, T + 1, T, 0, ng);
+                a.qlo = 1;
+                a.first = true;
+                CU(c, cudaEventRecord(c->ev0, c->st));
+                launch_res_fwd(s, c->dg, f, c->st);
+                launch_res_adj(s, c->dg, a, c->st);
+                CU(c, cudaEventRecord(c->ev1, c->st));
+                CU(c, cudaEventSynchronize(c->ev1));
+                CU(c, cudaGetLastError());
+                float t = 0.f;
+                CU(c, cudaEventElapsedTime(&t, c->ev0, c->ev1));
+                if (pass > 0) ms = std::min(ms, t);
+            }
+            if (tlog)
+                std::fprintf(stderr, "tomo tune: resident, %d groups: clusters of %d, %d warps of %d rows: %.2f us per %d steps\n",
+                             ng, s.cs, s.warps, s.rpw, 1e3 * ms, T);
+            if (ms < best) {
+                best = ms;
+                (which == 0 ? c->res1 : c->res) = s;
+            }
+        }
+        if (which == 0) c->res = c->res1;
+    }
+    if (cache && *cache)
+        if (FILE* fp = std::fopen(cache, "a")) {
+            std::fprintf(fp, "%s %d %d %d %d\n", key, c->res.cs, c->res.rpw, c->res1.cs, c->res1.rpw);
+            std::fclose(fp);
+        }
+    return TOMO_OK;
+}
+
 tomo_status run_pass(tomo_ctx* c, int mode, int g0, int ng) {
     const auto key = std::make_tuple(mode, g0, ng);
     auto it = c->graphs.find(key);
     if (it == c->graphs.end()) {
-        TRY(autotune(c));
+        if (!c->res.cpl || mode == MODE_ILLUM) TRY(autotune(c));
+        else TRY(tune_resident(c));
         LayoutScope layout(c, pass_layout(c, mode, ng));
         cudaGraph_t graph = nullptr;
         CU(c, cudaStreamBeginCapture(c->st, cudaStreamCaptureModeThreadLocal));
@@ -1127,7 +1356,7 @@ tomo_status apply_plan(tomo_ctx* c, const Plan& p) {
     c->release(&c->ckpt);
     c->release(&c->rr);
     set_plan(c, p);
-    c->tuned = false;
+    c->tuned = c->res_tuned = false;
     ++c->gen;
     TRY(alloc_plan_buffers(c));
     encode_maps(c);
@@ -1453,9 +1682,10 @@ tomo_status iterate_batch_graph(tomo_ctx** ctxs, int n, int method, const tomo_s
     // kernel choices first: the autotuner times trial passes, which a recording cannot hold
     for (int i = 0; i < n; ++i) {
         tomo_ctx* c = ctxs[i];
-        if (!c->tuned) {
+        if (c->res.cpl ? !c->res_tuned : !c->tuned) {
             launch_coef(c->geo.cfg.profile, c->f, c->coef, c->rcoef, c->geo.N, c->geo.cfg.courant, c->st);
-            TRY(autotune(c));
+            if (c->res.cpl) TRY(tune_resident(c));
+            else TRY(autotune(c));
         }
     }
     uint64_t sbits = 0;
@@ -2130,13 +2360,29 @@ tomo_status tomo_time_kernel(tomo_ctx* c, int32_t which, int32_t steps, double* 
     steps = std::min(steps, nt - 4);
     const int k0 = std::max(2, (nt - steps) / 2);
     launch_coef(prof, c->f, c->coef, c->rcoef, N, g.cfg.courant, c->st);
-    TRY(autotune(c));
+    if (!c->res.cpl) TRY(autotune(c));
+    else TRY(tune_resident(c));
     // the steps are captured into a graph and replayed, as the iterations run them, so the time
     // per step carries the launch gaps of graph replay, not of stream launches
     cudaGraph_t graph = nullptr;
     CU(c, cudaStreamBeginCapture(c->st, cudaStreamCaptureModeThreadLocal));
     for (int t = 0; t < steps;) {
-        if (which == 0 && c->tile_fwd) {
+        if (c->res.cpl) {   // a chunk of steps per launch, with the history traffic of a sweep
+            const ResShape& s = ng == 1 ? c->res1 : c->res;
+            const int T = std::min(steps - t, c->K);
+            if (which == 0) {
+                ResFwd f = res_fwd_args(c, s, k0, T, 0, ng);
+                f.hist = c->hist;
+                f.qlo = k0;
+                launch_res_fwd(s, c->dg, f, c->st);
+            } else {
+                ResAdj a = res_adj_args(c, s, k0 + T, T, 0, ng);
+                a.qlo = k0;
+                a.first = true;
+                launch_res_adj(s, c->dg, a, c->st);
+            }
+            t += T;
+        } else if (which == 0 && c->tile_fwd) {
             const int T = tile_fwd_steps(c, steps - t);
             launch_fwd_tile(c->dg, c->tmaps, tile_fwd_args(c, k0 + t, T, 0, ng), c->st);
             t += T;

@@ -315,6 +315,68 @@ void launch_fwd_tile(const DevGeo& g, const TileMaps& m, const TileFwd& a, void*
 void launch_adj_tile(const DevGeo& g, const TileMaps& m, const TileAdj& a, void* stream);
 // Whether a persistent (cooperative) launch of ng groups keeps every block resident at once.
 bool tile_persistent_fits(const DevGeo& g, int warps, bool fwd, int ng);
+// ---- cluster-resident sweeps (resident.cuh): CFG profile, wavefield in registers ---------------
+// A launch advances every group of a pass through a whole segment of time steps; a cluster of cs
+// blocks of `warps` warps holds one group.  Slices in memory are in fragment order (ns floats).
+struct ResShape {
+    int cpl = 0;         // cells per lane and row: a warp spans 32 cpl columns (0: not resident)
+    int rpw = 0;         // grid rows per warp
+    int warps = 0;       // warps per block
+    int cs = 0;          // blocks per cluster
+    int nrec = 0;        // receivers of the band that has most
+    int rows() const { return warps * rpw; }
+};
+struct ResFwd {
+    const float* coef;              // CFG coefficient, natural order
+    const float *in0, *in1;         // slices u(k0-1), u(k0) of pass-group 0, fragment order (null: zero)
+    int64_t instride;
+    int k0, T;                      // computes slices k0+1 .. k0+T
+    int g0, ng, cs;
+    float* hist;                    // L(q), q >= qlo, to slot q - qlo (null: none)
+    int64_t hstride, ns;            // floats between groups; per slice
+    int qlo;
+    float* ckpt;                    // checkpoints of the sweep (null: none): chunk ch >= 1 keeps the two
+    int64_t ckstride;               // slices up to res_restart(k0, K, ch)
+    int K, nchunk;
+    const float* gmeas;             // measured records of pass-group 0 (null: simulate)
+    float* gout;                    // records / residual (null: none)
+    const int32_t *rchan, *rcell, *rowstart;   // receivers in row order; first receiver of each row
+    float* out;                     // u(k0+T) in natural order (null: none)
+    int64_t outstride;
+    TileWait w;
+};
+struct ResAdj {
+    const float* coef;
+    const float* hist;              // L(q) at slot q - qlo, fragment order
+    int64_t hstride, ns;
+    int qlo;
+    const float* rr;                // residual records of pass-group 0: step m at rr + m * nch
+    int64_t rrstride;
+    const int32_t *rchan, *rcell, *rowstart;
+    float* st;                      // state of pass-group 0: z(kz0+1), z(kz0+2), correlation
+    int64_t ststride;
+    float* corr;                    // correlation of pass-group 0, natural order
+    int64_t cstride;
+    int kz0, T;                     // computes z(kz0) .. z(kz0-T+1)
+    int ng, cs;
+    bool first, last;               // sweep's first launch (state zero) / last (writes corr)
+    TileWait w;
+};
+// Cells per lane for grids of nx columns (0: too wide to stay on chip), and the floats of a slice in
+// fragment order.
+int res_width(int nx);
+int64_t res_slice(int nx, int ny);
+// Every cluster shape that takes a group of an nx x ny grid (none: the grid does not fit on chip), and
+// the clusters of a shape this GPU holds at once (0: it cannot run the shape).
+int res_held(const ResShape& s);
+std::vector<ResShape> res_shapes(int nx, int ny, const std::vector<int32_t>& rowstart);
+// Newest of the two slices that chunk ch of a sweep from slice k0, cut every K slices, restarts from.
+int res_restart(int k0, int K, int ch);
+// Receivers in row order (channel and cell), and the first of each row (ny + 1 entries).
+void res_receivers(const std::vector<int32_t>& rcv, int nx, int ny, std::vector<int32_t>& chan,
+                   std::vector<int32_t>& cell, std::vector<int32_t>& rowstart);
+void launch_res_fwd(const ResShape& s, const DevGeo& g, const ResFwd& a, void* stream);
+void launch_res_adj(const ResShape& s, const DevGeo& g, const ResAdj& a, void* stream);
 // cuTensorMapEncodeTiled, looked up from the driver once (no link against libcuda); null when
 // the driver has none.
 void* tensor_map_encoder();

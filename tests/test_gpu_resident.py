@@ -74,6 +74,44 @@ def test_resident_matches_per_step_kernels(name, monkeypatch):
     assert np.abs(got[0]).max() > 0
 
 
+# reference profile: rows between the paired ones even and odd in number, the smallest ring margin,
+# non-square grids, right edges at each place of a lane, emission boxes around a corner
+REF = {
+    "64x60": dict(nx=64, ny=60, nt=150, ring_lo=8, ring_hi=50, group_size=24),
+    "odd, checkpoints of 9": dict(nx=61, ny=53, nt=131, ring_lo=7, ring_hi=44, group_size=20, ckpt_interval=9,
+                                  groups_per_pass=3),
+    "least margin, checkpoints of 2": dict(nx=97, ny=98, nt=110, ring_lo=2, ring_hi=94, group_size=60, ckpt_interval=2),
+    "smallest ring": dict(nx=22, ny=23, nt=90, ring_lo=8, ring_hi=11, group_size=4),
+    "ring of two (per-step kernels)": dict(nx=24, ny=24, nt=60, ring_lo=10, ring_hi=12, group_size=4),
+    "192": dict(nx=192, ny=192, nt=401, ring_lo=20, ring_hi=180, group_size=80),
+    "195x130": dict(nx=195, ny=130, nt=160, ring_lo=11, ring_hi=117, group_size=100, ckpt_interval=33),
+    "288": dict(nx=288, ny=288, nt=120, ring_lo=30, ring_hi=257, group_size=227),
+}
+
+
+@pytest.mark.parametrize("name", sorted(REF))
+def test_reference_profile_matches_per_step_kernels(name, monkeypatch):
+    cfg = tomo.ref_config(**REF[name])
+    fo = 0.4 * phantom(cfg)
+    got = sweep(cfg, fo)
+    monkeypatch.setenv("TOMO_RESIDENT", "0")
+    want = sweep(cfg, fo)
+    for k, (a, b) in enumerate(zip(got, want)):
+        assert np.array_equal(a, b, equal_nan=True), (name, k, rel(a, b))
+    assert np.abs(got[0]).max() > 0
+
+
+@pytest.mark.parametrize("shape", ["16,2", "13,2", "7,2"])
+def test_every_reference_cluster_shape_gives_the_same_bits(shape, monkeypatch):
+    cfg = tomo.ref_config(nx=118, ny=119, nt=140, ring_lo=13, ring_hi=104, group_size=91, ckpt_interval=21)
+    fo = 0.4 * phantom(cfg)
+    want = sweep(cfg, fo)
+    monkeypatch.setenv("TOMO_RES_SHAPE", shape)
+    got = sweep(cfg, fo)
+    for k, (a, b) in enumerate(zip(got, want)):
+        assert np.array_equal(a, b), (shape, k, rel(a, b))
+
+
 @pytest.mark.parametrize("shape", ["16,1", "7,1", "16,2", "5,2", "4,4", "11,4"])
 def test_every_cluster_shape_gives_the_same_bits(shape, monkeypatch):
     cfg = ring(nx=126, ny=111, nt=100, ns=30, gs=5, ckpt=13)
@@ -114,12 +152,16 @@ def test_resident_residual_noise(kind, monkeypatch):
     assert np.abs(outs[0]).max() > 0
 
 
-def test_row_that_never_arrives_is_a_status(monkeypatch):
+@pytest.mark.parametrize("profile", ["ring", "reference"])
+def test_row_that_never_arrives_is_a_status(profile, monkeypatch):
     """A cluster whose barriers expect bytes that never come gives up after the wait limit: the call
     returns TOMO_ERR_TIMEOUT, and a context made afterwards works."""
-    cfg = ring(nx=96, ny=96, nt=80, ns=16, gs=8)
+    if profile == "ring":
+        cfg = ring(nx=96, ny=96, nt=80, ns=16, gs=8)
+    else:
+        cfg = tomo.ref_config(nx=64, ny=60, nt=60, ring_lo=8, ring_hi=50, group_size=42)
     fo = phantom(cfg)
-    monkeypatch.setenv("TOMO_RES_SHAPE", "4,4")
+    monkeypatch.setenv("TOMO_RES_SHAPE", "4,4" if profile == "ring" else "4,2")
     monkeypatch.setenv("TOMO_WAIT_LIMIT_NS", "2000000")
     monkeypatch.setenv("TOMO_TEST_UNDELIVERED_TX", "16")
     with tomo.Context(cfg) as ctx:
@@ -129,4 +171,6 @@ def test_row_that_never_arrives_is_a_status(monkeypatch):
     monkeypatch.delenv("TOMO_TEST_UNDELIVERED_TX")
     with tomo.Context(cfg) as ctx:
         rec = ctx.forward(fo)
-    assert rel(rec, O.forward(cfg, fo.astype(np.float64))) <= TOL_WAVE
+    monkeypatch.setenv("TOMO_RESIDENT", "0")
+    with tomo.Context(cfg) as ctx:
+        assert np.array_equal(rec, ctx.forward(fo))

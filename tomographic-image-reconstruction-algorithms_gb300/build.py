@@ -25,7 +25,7 @@ ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 COMMON = ["-O3", "-std=c++17", "-lineinfo", "-I" + INCLUDE, "-I" + CSRC]
 
 LIB_SOURCES = ["kernels.cu", "strip.cu", "tile.cu", "resident.cu", "resident_a.cu", "resident_b.cu",
-               "resident_c.cu", "resident_d.cu", "engine.cu", "geometry.cpp", "noalloc.cu", "cnn.cu", "net.cu"]
+               "resident_c.cu", "resident_d.cu", "resident_e.cu", "resident_f.cu", "engine.cu", "geometry.cpp", "noalloc.cu", "cnn.cu", "net.cu"]
 # driver name -> -D selector of cli/tomo_cli.cpp
 DRIVERS = {
     "generate-field": "GENERATE_FIELD",
@@ -46,7 +46,7 @@ DRIVERS = {
     "tomo": "TOMO_MULTI",
 }
 HEADERS = [os.path.join(INCLUDE, "tomo.h"), os.path.join(CSRC, "internal.h"), os.path.join(CSRC, "cell.cuh"),
-           os.path.join(CSRC, "async.cuh"), os.path.join(CSRC, "resident.cuh"), os.path.join(CSRC, "cnn.h")]
+           os.path.join(CSRC, "async.cuh"), os.path.join(CSRC, "resident.cuh"), os.path.join(CSRC, "resident_ref.cuh"), os.path.join(CSRC, "cnn.h")]
 
 
 def _newer(target: str, deps: list[str]) -> bool:

@@ -87,7 +87,8 @@ struct tomo_ctx {
     ResShape res, res1;
     int64_t NS = 0;
     int32_t *rchan = nullptr, *rcell = nullptr, *rowstart = nullptr;
-    std::vector<int32_t> h_rowstart;
+    std::vector<int32_t> h_rowstart, h_warps;
+    int32_t *warps = nullptr, *rowslot = nullptr;   // reference profile: rows of each warp, slot of each row
     std::vector<ResShape> res_cands;   // every shape that holds a group (tune_resident times them)
     bool res_tuned = false;
     // learned iteration (allocated on first use)
@@ -661,16 +662,21 @@ void choose_resident(tomo_ctx* c) {
     const Geometry& g = c->geo;
     c->NS = g.N;
     const char* e = std::getenv("TOMO_RESIDENT");
-    if (g.ref || (e && *e == '0') || std::getenv("TOMO_STRIP_ROWS") || std::getenv("TOMO_TILE") ||
+    if ((e && *e == '0') || std::getenv("TOMO_STRIP_ROWS") || std::getenv("TOMO_TILE") ||
         std::getenv("TOMO_NO_STRIP"))
         return;
     std::vector<int32_t> chan, cell;
     res_receivers(g.rcv, g.nx, g.ny, chan, cell, c->h_rowstart);
-    c->res_cands = res_shapes(g.nx, g.ny, c->h_rowstart);
+    if (g.ref) {
+        c->h_warps = ref_warps(g.ny, g.lo, g.hi);
+        c->res_cands = ref_shapes(g.nx, g.ny, c->h_warps, c->h_rowstart);
+    } else {
+        c->res_cands = res_shapes(g.nx, g.ny, c->h_rowstart);
+    }
     while (!c->res_cands.empty() && res_held(c->res_cands.back()) < 1) c->res_cands.pop_back();
     if (c->res_cands.empty()) return;
     c->res = c->res1 = c->res_cands.back();   // tune_resident picks among them
-    c->NS = res_slice(g.nx, g.ny);
+    c->NS = res_slice(c->res, g.ny);
 }
 
 // Chosen memory plan.  ckpt_interval > 0 fixes K; 0 and -1 start from full history when it fits
@@ -748,7 +754,16 @@ tomo_status create_buffers(tomo_ctx* c) {
         CU(c, cudaMemcpyAsync(c->rcell, cell.data(), sizeof(int32_t) * cell.size(), cudaMemcpyHostToDevice, c->st));
         CU(c, cudaMemcpyAsync(c->rowstart, c->h_rowstart.data(), sizeof(int32_t) * c->h_rowstart.size(),
                               cudaMemcpyHostToDevice, c->st));
-        TRY(sync_check(c));   // `chan` and `cell` are local
+        std::vector<int32_t> slot((size_t)g.ny, 0);
+        for (size_t w = 0; w < c->h_warps.size(); ++w)
+            for (int r = 0; r < c->h_warps[w] >> 16; ++r) slot[(c->h_warps[w] & 0xffff) + r] = (int32_t)(2 * w) + r;
+        if (!c->h_warps.empty()) {
+            TRY(c->alloc(&c->warps, (int64_t)c->h_warps.size(), "warp rows"));
+            TRY(c->alloc(&c->rowslot, g.ny, "row slots"));
+            CU(c, cudaMemcpyAsync(c->warps, c->h_warps.data(), sizeof(int32_t) * c->h_warps.size(), cudaMemcpyHostToDevice, c->st));
+            CU(c, cudaMemcpyAsync(c->rowslot, slot.data(), sizeof(int32_t) * g.ny, cudaMemcpyHostToDevice, c->st));
+        }
+        TRY(sync_check(c));   // `chan`, `cell` and `slot` are local
     }
     if (g.ref) TRY(c->alloc(&c->box, 4 * G, "boxes"));
     else {
@@ -829,6 +844,10 @@ ResFwd res_fwd_args(tomo_ctx* c, const ResShape& s, int k0, int T, int g0, int n
     a.rchan = c->rchan;
     a.rcell = c->rcell;
     a.rowstart = c->rowstart;
+    a.rcoef = c->rcoef;
+    a.warps = c->warps;
+    a.rowslot = c->rowslot;
+    a.nwarps = (int)c->h_warps.size();
     a.w = TileWait{c->err_dev, c->wait_ns, c->test_tx, c->gbar, c->test_gbar};
     return a;
 }
@@ -845,6 +864,9 @@ ResAdj res_adj_args(tomo_ctx* c, const ResShape& s, int kz0, int T, int g0, int 
     a.rchan = c->rchan;
     a.rcell = c->rcell;
     a.rowstart = c->rowstart;
+    a.field = c->f;
+    a.warps = c->warps;
+    a.nwarps = (int)c->h_warps.size();
     a.st = c->z;
     a.ststride = tomo_ctx::ZR * c->NS;
     a.corr = c->corr + (int64_t)g0 * c->geo.N;
@@ -902,7 +924,7 @@ int64_t record_resident_pass(tomo_ctx* c, int mode, int g0, int ng) {
             launch_res_fwd(s, c->dg, r, c->st);
             ++n;
         }
-        ResAdj a = res_adj_args(c, s, qb + 1, T, g0, ng);
+        ResAdj a = res_adj_args(c, s, g.ref ? qb : qb + 1, T, g0, ng);   // the slice of z paired with L(qb)
         a.qlo = qa;
         a.first = ch == c->nchunk - 1;
         a.last = ch == 0;
@@ -1210,7 +1232,7 @@ tomo_status tune_resident(tomo_ctx* c) {
     const Geometry& g = c->geo;
     const char* cache = std::getenv("TOMO_TUNE_CACHE");
     char key[160];
-    std::snprintf(key, sizeof key, "tomo-res-1 %d %d %d %d %d", g.nx, g.ny, g.nt, c->P, c->S);
+    std::snprintf(key, sizeof key, "tomo-res-1 %d %d %d %d %d %d", g.cfg.profile, g.nx, g.ny, g.nt, c->P, c->S);
     if (cache && *cache)
         if (FILE* fp = std::fopen(cache, "r")) {
             char line[512];
@@ -1243,7 +1265,7 @@ tomo_status tune_resident(tomo_ctx* c) {
                 ResFwd f = res_fwd_args(c, s, 1, T, 0, ng);
                 f.hist = c->hist;
                 f.qlo = 1;
-                ResAdj a = res_adj_args(c, s, T + 1, T, 0, ng);
+                ResAdj a = res_adj_args(c, s, g.ref ? T : T + 1, T, 0, ng);
                 a.qlo = 1;
                 a.first = true;
                 CU(c, cudaEventRecord(c->ev0, c->st));
@@ -2376,7 +2398,7 @@ tomo_status tomo_time_kernel(tomo_ctx* c, int32_t which, int32_t steps, double* 
                 f.qlo = k0;
                 launch_res_fwd(s, c->dg, f, c->st);
             } else {
-                ResAdj a = res_adj_args(c, s, k0 + T, T, 0, ng);
+                ResAdj a = res_adj_args(c, s, g.ref ? k0 + T - 1 : k0 + T, T, 0, ng);
                 a.qlo = k0;
                 a.first = true;
                 launch_res_adj(s, c->dg, a, c->st);

@@ -315,10 +315,11 @@ void launch_fwd_tile(const DevGeo& g, const TileMaps& m, const TileFwd& a, void*
 void launch_adj_tile(const DevGeo& g, const TileMaps& m, const TileAdj& a, void* stream);
 // Whether a persistent (cooperative) launch of ng groups keeps every block resident at once.
 bool tile_persistent_fits(const DevGeo& g, int warps, bool fwd, int ng);
-// ---- cluster-resident sweeps (resident.cuh): CFG profile, wavefield in registers ---------------
+// ---- cluster-resident sweeps (resident.cuh, resident_ref.cuh): wavefield in registers -----------
 // A launch advances every group of a pass through a whole segment of time steps; a cluster of cs
 // blocks of `warps` warps holds one group.  Slices in memory are in fragment order (ns floats).
 struct ResShape {
+    bool ref = false;    // reference-profile sweeps
     int cpl = 0;         // cells per lane and row: a warp spans 32 cpl columns (0: not resident)
     int rpw = 0;         // grid rows per warp
     int warps = 0;       // warps per block
@@ -341,6 +342,9 @@ struct ResFwd {
     const float* gmeas;             // measured records of pass-group 0 (null: simulate)
     float* gout;                    // records / residual (null: none)
     const int32_t *rchan, *rcell, *rowstart;   // receivers in row order; first receiver of each row
+    const float* rcoef;             // reference profile: velocity; rows of each warp, slot of each row
+    const int32_t *warps, *rowslot;
+    int nwarps;
     float* out;                     // u(k0+T) in natural order (null: none)
     int64_t outstride;
     TileWait w;
@@ -353,6 +357,9 @@ struct ResAdj {
     const float* rr;                // residual records of pass-group 0: step m at rr + m * nch
     int64_t rrstride;
     const int32_t *rchan, *rcell, *rowstart;
+    const float* field;             // reference profile: the field f; rows of each warp
+    const int32_t* warps;
+    int nwarps;
     float* st;                      // state of pass-group 0: z(kz0+1), z(kz0+2), correlation
     int64_t ststride;
     float* corr;                    // correlation of pass-group 0, natural order
@@ -362,14 +369,15 @@ struct ResAdj {
     bool first, last;               // sweep's first launch (state zero) / last (writes corr)
     TileWait w;
 };
-// Cells per lane for grids of nx columns (0: too wide to stay on chip), and the floats of a slice in
-// fragment order.
-int res_width(int nx);
-int64_t res_slice(int nx, int ny);
 // Every cluster shape that takes a group of an nx x ny grid (none: the grid does not fit on chip), and
 // the clusters of a shape this GPU holds at once (0: it cannot run the shape).
 int res_held(const ResShape& s);
 std::vector<ResShape> res_shapes(int nx, int ny, const std::vector<int32_t>& rowstart);
+int64_t res_slice(const ResShape& s, int ny);   // floats of a slice in fragment order
+// Reference profile: the rows of each warp (first row, count in the high half; empty: not resident), and
+// the shapes that take them.
+std::vector<int32_t> ref_warps(int ny, int lo, int hi);
+std::vector<ResShape> ref_shapes(int nx, int ny, const std::vector<int32_t>& warps, const std::vector<int32_t>& rowstart);
 // Newest of the two slices that chunk ch of a sweep from slice k0, cut every K slices, restarts from.
 int res_restart(int k0, int K, int ch);
 // Receivers in row order (channel and cell), and the first of each row (ny + 1 entries).

@@ -9,7 +9,7 @@
 
 namespace tomo {
 
-#define RES_WIDTHS(X) X(a) X(b) X(c) X(d)
+#define RES_WIDTHS(X) X(a) X(b) X(c) X(d) X(e) X(f)
 #define RES_DECL(W)                                                                                        \
     cudaError_t res_fwd_##W(const ResShape& s, const DevGeo* g, const ResFwd* a, int* held, void* stream); \
     cudaError_t res_adj_##W(const ResShape& s, const DevGeo* g, const ResAdj* a, int* held, void* stream);
@@ -30,10 +30,12 @@ int cells_per_lane(int nx) {
     return 0;
 }
 cudaError_t fwd(const ResShape& s, const DevGeo* g, const ResFwd* a, int* held, void* st) {
+    if (s.ref) return s.cpl <= 6 ? res_fwd_e(s, g, a, held, st) : res_fwd_f(s, g, a, held, st);
     return s.cpl <= 4 ? res_fwd_a(s, g, a, held, st) : s.cpl <= 8 ? res_fwd_b(s, g, a, held, st)
          : s.cpl <= 12 ? res_fwd_c(s, g, a, held, st) : res_fwd_d(s, g, a, held, st);
 }
 cudaError_t adj(const ResShape& s, const DevGeo* g, const ResAdj* a, int* held, void* st) {
+    if (s.ref) return s.cpl <= 6 ? res_adj_e(s, g, a, held, st) : res_adj_f(s, g, a, held, st);
     return s.cpl <= 4 ? res_adj_a(s, g, a, held, st) : s.cpl <= 8 ? res_adj_b(s, g, a, held, st)
          : s.cpl <= 12 ? res_adj_c(s, g, a, held, st) : res_adj_d(s, g, a, held, st);
 }
@@ -46,8 +48,51 @@ int band_receivers(const std::vector<int32_t>& rowstart, int ny, int rows) {
 }
 }  // namespace
 
-int res_width(int nx) { return cells_per_lane(nx); }
-int64_t res_slice(int nx, int ny) { return (int64_t)32 * cells_per_lane(nx) * ny; }
+int64_t res_slice(const ResShape& s, int ny) { return (int64_t)32 * s.cpl * ny; }
+
+// Reference profile: cells per lane of a width (0: too wide).
+static int ref_cells_per_lane(int nx) {
+    for (const int c : {4, 6, 8, 10})
+        if (nx <= 32 * c) return c;
+    return 0;
+}
+
+std::vector<int32_t> ref_warps(int ny, int lo, int hi) {
+    std::vector<int32_t> out;
+    if (lo < 2 || hi < lo + 3 || hi > ny - 3) return out;   // the paired rows must be four distinct pairs
+    auto rows = [&](int a, int b) {                          // rows a .. b-1: pairs, an odd one alone
+        for (int j = a; j < b; j += 2) out.push_back(j | (std::min(2, b - j) << 16));
+    };
+    rows(0, 2);
+    rows(2, lo);
+    rows(lo, lo + 2);
+    rows(lo + 2, hi - 1);
+    rows(hi - 1, hi + 1);
+    rows(hi + 1, ny - 2);
+    rows(ny - 2, ny);
+    return out;
+}
+
+std::vector<ResShape> ref_shapes(int nx, int ny, const std::vector<int32_t>& warps, const std::vector<int32_t>& rowstart) {
+    std::vector<ResShape> out;
+    const int cpl = ref_cells_per_lane(nx), nw = (int)warps.size();
+    if (cpl == 0 || nw == 0 || ny > 0x7fff) return out;
+    for (int cs = kMaxCluster; cs >= 1; --cs) {
+        ResShape s;
+        s.ref = true;
+        s.cpl = cpl;
+        s.rpw = 2;
+        s.cs = cs;
+        s.warps = (nw + cs - 1) / cs;
+        if (s.warps > 16 || s.warps * (cs - 1) >= nw) continue;
+        for (int b = 0; b < cs; ++b) {
+            const int first = warps[b * s.warps], last = warps[std::min(nw, (b + 1) * s.warps) - 1];
+            s.nrec = std::max(s.nrec, rowstart[(last & 0xffff) + (last >> 16)] - rowstart[first & 0xffff]);
+        }
+        out.push_back(s);
+    }
+    return out;
+}
 int res_restart(int k0, int K, int ch) { return ch * K + 1 - ((ch * K + 1 - k0) & 1); }
 
 std::vector<ResShape> res_shapes(int nx, int ny, const std::vector<int32_t>& rowstart) {

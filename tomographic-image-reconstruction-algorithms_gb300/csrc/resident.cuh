@@ -253,6 +253,7 @@ template <int CPL>
 struct ResLinks {
     uint32_t lo_row, lo_bar, hi_row, hi_bar;   // remote addresses, parity 0
     uint64_t limit_ns;
+    bool single = false;                       // the warp's only row is its first
     bool lo, hi;                               // link open: this warp has the block's first / last row, a neighbour beyond
     __device__ __forceinline__ void init(const ResSmem& sm, int rank, int cs, bool first, bool last, uint64_t limit) {
         constexpr int ROW = 32 * CPL;
@@ -269,7 +270,8 @@ struct ResLinks {
     __device__ __forceinline__ void send(const float2 (&first)[CPL / 2], const float2 (&last)[CPL / 2], int lane) const {
         constexpr uint32_t step = 4u * 32u * CPL;
         if (lo) Frag<CPL>::send(lo_row + P * step, lo_bar + 8u * P, first, lane);
-        if (hi) Frag<CPL>::send(hi_row + P * step, hi_bar + 8u * P, last, lane);
+        if (hi && !single) Frag<CPL>::send(hi_row + P * step, hi_bar + 8u * P, last, lane);
+        if (hi && single) Frag<CPL>::send(hi_row + P * step, hi_bar + 8u * P, first, lane);
     }
     // Row t - 1 of parity P.  A wait that runs out is noted for res_failed; the block then leaves.
     template <int P, bool ARM = true>

@@ -1,0 +1,22 @@
+// resident_f.cu -- instantiations of the cluster-resident reference-profile sweeps
+// (resident_ref.cuh) for 8 and 10 cells per lane.
+#include "resident_ref.cuh"
+
+namespace tomo {
+namespace {
+template <typename Args>
+cudaError_t pick(const ResShape& s, const DevGeo* g, const Args* a, int* held, void* stream) {
+    if (s.cpl == 8) return ref_go<8>(s, g, a, held, stream);
+    if (s.cpl == 10) return ref_go<10>(s, g, a, held, stream);
+    return cudaErrorInvalidValue;
+}
+}  // namespace
+
+cudaError_t res_fwd_f(const ResShape& s, const DevGeo* g, const ResFwd* a, int* held, void* stream) {
+    return pick(s, g, a, held, stream);
+}
+cudaError_t res_adj_f(const ResShape& s, const DevGeo* g, const ResAdj* a, int* held, void* stream) {
+    return pick(s, g, a, held, stream);
+}
+
+}  // namespace tomo

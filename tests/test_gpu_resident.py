@@ -174,3 +174,27 @@ def test_row_that_never_arrives_is_a_status(profile, monkeypatch):
     monkeypatch.setenv("TOMO_RESIDENT", "0")
     with tomo.Context(cfg) as ctx:
         assert np.array_equal(rec, ctx.forward(fo))
+
+
+@pytest.mark.parametrize("cfg", [
+    ring(nx=72, ny=64, nt=180, ns=24, gs=4), ring(nx=61, ny=47, nt=90, ns=16, gs=4), ring(nx=250, ny=190, nt=60, ns=60, gs=2),
+    ring(nx=400, ny=396, nt=60, ns=16, gs=8), ring(nx=401, ny=397, nt=40, ns=16, gs=8),   # strips; per-cell
+    tomo.ref_config(nx=61, ny=53, nt=100, ring_lo=7, ring_hi=44, group_size=2),
+    tomo.ref_config(nx=340, ny=330, nt=40, ring_lo=20, ring_hi=300, group_size=280),     # per-cell
+], ids=lambda c: f"{'reference' if c.profile == tomo.PROFILE_REF else 'ring'}-{c.nx}x{c.ny}")
+def test_allocation_free_forward_has_the_same_bits(cfg):
+    import ctypes as C
+
+    import torch
+
+    fo = (0.4 if cfg.profile == tomo.PROFILE_REF else 1.0) * phantom(cfg)
+    with tomo.Context(cfg) as ctx:
+        want = ctx.forward(fo)
+    d_f = torch.from_numpy(fo.astype(np.float32)).cuda()
+    d_rec = torch.full(want.shape, -1.0, device="cuda")
+    torch.cuda.synchronize()
+    for _ in range(2):
+        assert tomo.lib().tomo_forward_noalloc(C.byref(cfg), C.c_void_p(d_f.data_ptr()), C.c_void_p(d_rec.data_ptr()),
+                                               None) == tomo.OK
+    torch.cuda.synchronize()
+    assert np.array_equal(d_rec.cpu().numpy(), want)

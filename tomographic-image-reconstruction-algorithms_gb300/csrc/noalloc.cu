@@ -8,10 +8,15 @@
 // streams.  They pass their own input and output buffers; the wavefield
 // scratch this solve needs lives in the file-scope array below instead.
 //
+// Grids that fit on chip (resident.cuh) are solved by one launch for all groups, which keeps the
+// wavefield in registers and uses the array for the coefficients and tables only: 128 x 128, 600
+// steps, 8 groups took 39.2 ms as a step and a gather launch per time step and group.  Larger grids
+// go a group at a time through the array's time slots.
+//
 // The scratch array g_scratch is a fixed kNoallocScratchBytes (about 5.1 MiB)
-// that every GPU loading this library holds until the process exits.  It holds,
-// for one emitter group at a time, the three forward time slots, the two
-// coefficient fields and the geometry tables, so a call accepts grids of up to
+// that every GPU loading this library holds until the process exits.  It holds
+// the two coefficient fields, the geometry tables and, for one emitter group at
+// a time, three forward time slots, so a call accepts grids of up to
 // kNoallocMaxCells cells (512 x 512), kNoallocMaxChannels record channels and
 // kNoallocMaxSteps time steps, plus kNoallocMaxEmitters emitters (benchmark
 // profile) or kNoallocMaxGroups emission boxes (reference profile), and rejects
@@ -35,10 +40,12 @@
 // serialise them on one stream.
 #include <cuda_runtime.h>
 
-#include <cstdio>
-#include <cstring>
 #include <algorithm>
+#include <cstdio>
+#include <cstdlib>
+#include <cstring>
 #include <string>
+#include <vector>
 
 #include "internal.h"
 
@@ -50,18 +57,20 @@ constexpr int kNoallocMaxChannels = 2048;
 constexpr int kNoallocMaxGroups = 2048;
 constexpr int kNoallocMaxEmitters = 4096;
 constexpr int kNoallocMaxSteps = 16384;
+constexpr int kNoallocMaxRows = 1024;      // grid rows of a cluster-resident solve
 
 // float region: 3 time slots + coefficient + edge coefficient + source table
 constexpr int64_t kFloats = 5 * kNoallocMaxCells + kNoallocMaxSteps;
-// int region: receiver cells + emitter cells + emission boxes
-constexpr int64_t kInts = kNoallocMaxChannels + kNoallocMaxEmitters + 4 * kNoallocMaxGroups;
+// int region: receiver cells, emitter cells, emission boxes; for a cluster-resident solve receivers in row
+// order (channel, cell), the first of each row, and the reference profile's rows of each warp and row slots
+constexpr int64_t kInts = 3 * kNoallocMaxChannels + kNoallocMaxEmitters + 4 * kNoallocMaxGroups + 3 * (kNoallocMaxRows + 1);
 constexpr int64_t kNoallocScratchBytes = 4 * (kFloats + kInts);
 
 static __device__ __align__(256) unsigned char g_scratch[kNoallocScratchBytes];
 
-// Words of table data carried by one k_put_words launch (the argument block stays under the
-// 4 KB kernel-parameter limit of every CUDA version).
-constexpr int kWordsPerLaunch = 1000;
+// Words of table data carried by one k_put_words launch (the argument block stays under the 32764-byte
+// kernel-parameter limit): most problems' tables go in one launch.
+constexpr int kWordsPerLaunch = 4000;
 struct Words {
     uint32_t v[kWordsPerLaunch];
 };
@@ -129,47 +138,104 @@ extern "C" tomo_status tomo_forward_noalloc(const tomo_config* cfg, const float*
     float* slots = (float*)base;                       // 3 time slots
     float* coef = slots + 3 * kNoallocMaxCells;
     float* rcoef = coef + kNoallocMaxCells;
-    float* src = rcoef + kNoallocMaxCells;
-    int32_t* rcv = (int32_t*)(src + kNoallocMaxSteps);
-    int32_t* emit = rcv + kNoallocMaxChannels;
-    int32_t* box = emit + kNoallocMaxEmitters;
+    float* src = rcoef + kNoallocMaxCells;             // tables: source, then the integer tables behind it
     cudaError_t e;
 #define NA_CU(x)                                     \
     do {                                             \
         if ((e = (x)) != cudaSuccess) return cuda_fail(e, #x); \
     } while (0)
-    if ((s = put_words((uint32_t*)src, geo.src.data(), (int64_t)geo.src.size(), st)) != TOMO_OK) return s;
-    if ((s = put_words((uint32_t*)rcv, geo.rcv.data(), nch, st)) != TOMO_OK) return s;
-    if (geo.ref) s = put_words((uint32_t*)box, geo.box.data(), 4 * (int64_t)geo.G, st);
-    else s = put_words((uint32_t*)emit, geo.emit.data(), (int64_t)geo.G * geo.gs, st);
-    if (s != TOMO_OK) return s;
-    NA_CU(cudaMemsetAsync(d_records, 0, sizeof(float) * (size_t)geo.G * nt * nch, st));
     DevGeo dg{};
     dg.nx = geo.nx; dg.ny = geo.ny; dg.nt = geo.nt; dg.nch = geo.nch;
     dg.lo = geo.lo; dg.hi = geo.hi; dg.gs = geo.gs;
     dg.sponge_w = cfg->sponge_width; dg.sponge_max = cfg->sponge_max;
     fill_damp(dg);
-    dg.box = box; dg.emit = emit; dg.rcv = rcv; dg.rid = nullptr; dg.rbits = nullptr; dg.rwords = 0; dg.src = src;
     dg.n_src_steps = geo.n_src_steps;
+    dg.src = src;
     const int prof = cfg->profile;
+    // a grid that fits on chip is solved by one launch for all groups
+    std::vector<int32_t> chan, cell, rowstart, warps, slot;
+    ResShape shape;
+    if (const char* off = std::getenv("TOMO_RESIDENT"); geo.ny <= kNoallocMaxRows && !(off && *off == '0')) {
+        res_receivers(geo.rcv, geo.nx, geo.ny, chan, cell, rowstart);
+        if (geo.ref) warps = ref_warps(geo.ny, geo.lo, geo.hi);
+        shape = res_pick(geo.ref ? ref_shapes(geo.nx, geo.ny, warps, rowstart) : res_shapes(geo.nx, geo.ny, rowstart), geo.G);
+        if (shape.cpl && res_held(shape) < 1) shape = ResShape{};
+    }
+    // every table in one block of words behind the source table
+    std::vector<uint32_t> words;
+    auto put = [&](const void* p, int64_t n) {         // returns the table's device address
+        const uint32_t* w = (const uint32_t*)p;
+        const int64_t at = (int64_t)words.size();
+        words.insert(words.end(), w, w + n);
+        return (int32_t*)src + at;
+    };
+    put(geo.src.data(), shape.cpl ? std::min<int64_t>((int64_t)geo.src.size(), geo.ref ? 2 * geo.n_src_steps : geo.n_src_steps)
+                                  : (int64_t)geo.src.size());
+    if (geo.ref) dg.box = put(geo.box.data(), 4 * (int64_t)geo.G);
+    else dg.emit = put(geo.emit.data(), (int64_t)geo.G * geo.gs);
+    ResFwd r{};
+    if (shape.cpl) {
+        r.rchan = put(chan.data(), (int64_t)chan.size());
+        r.rcell = put(cell.data(), (int64_t)cell.size());
+        r.rowstart = put(rowstart.data(), geo.ny + 1);
+        if (geo.ref) {
+            slot.assign((size_t)geo.ny, 0);
+            for (size_t w = 0; w < warps.size(); ++w)
+                for (int k = 0; k < warps[w] >> 16; ++k) slot[(warps[w] & 0xffff) + k] = (int32_t)(2 * w) + k;
+            r.warps = put(warps.data(), (int64_t)warps.size());
+            r.rowslot = put(slot.data(), geo.ny);
+            r.nwarps = (int)warps.size();
+        }
+    } else {
+        dg.rcv = put(geo.rcv.data(), nch);
+    }
+    // the word the kernels' bounded waits would set; nothing reads it
+    static const uint32_t zero = 0;
+    unsigned int* const err = (unsigned int*)put(&zero, 1);
+    if ((s = put_words((uint32_t*)src, words.data(), (int64_t)words.size(), st)) != TOMO_OK) return s;
+    NA_CU(cudaMemsetAsync(d_records, 0, sizeof(float) * (size_t)geo.G * nt * nch, st));
     launch_coef(prof, d_f, coef, rcoef, N, cfg->courant, st);
-    auto slot = [&](int k) { return slots + (int64_t)(k % 3) * N; };
+    if (shape.cpl) {
+        r.coef = coef;
+        r.rcoef = rcoef;
+        r.k0 = 1;
+        r.T = geo.nt - 2;
+        r.ng = geo.G;
+        r.cs = shape.cs;
+        r.gout = d_records;
+        r.w = TileWait{err, 1000000000ull, 0u, nullptr, 0u};
+        launch_res_fwd(shape, dg, r, st);
+        NA_CU(cudaGetLastError());
+        return TOMO_OK;
+    }
+    // otherwise a group at a time: a strip launch per step, which also gathers the slice before (widths of
+    // whole 128-bit vectors), or a step and a gather launch
+    const bool strip = !geo.ref && geo.nx % 4 == 0;   // k_fwd_strip reads none of the receiver maps
+    auto at = [&](int k) { return slots + (int64_t)(k % 3) * N; };
     for (int g = 0; g < geo.G; ++g) {
         launch_zero_slots(slots, 1, 3 * N, 0, N, N, st);   // u(0) = u(1) = 0
+        float* const out = d_records + (int64_t)g * nt * nch;
         for (int k = 1; k <= geo.nt - 2; ++k) {
             FwdStep fs{};
-            fs.up = slot(k - 1);
-            fs.uc = slot(k);
-            fs.un = slot(k + 1);
+            fs.up = at(k - 1);
+            fs.uc = at(k);
+            fs.un = at(k + 1);
             fs.gstride = 3 * N;
             fs.k = k;
             fs.g0 = g;
             fs.ng = 1;
-            launch_fwd_step(prof, dg, coef, rcoef, fs, st);
+            if (strip) {
+                fs.gk = k;
+                fs.gout = out;
+                launch_fwd_strip(8, dg, coef, fs, st);
+                if (k < geo.nt - 2) continue;
+            } else {
+                launch_fwd_step(prof, dg, coef, rcoef, fs, st);
+            }
             GatherStep gs{};
-            gs.u = slot(k + 1);
+            gs.u = at(k + 1);
             gs.gstride = 3 * N;
-            gs.out = d_records + (int64_t)g * nt * nch;
+            gs.out = out;
             gs.k = k + 1;
             gs.ng = 1;
             launch_gather(dg, gs, st);

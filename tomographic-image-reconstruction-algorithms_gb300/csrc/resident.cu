@@ -123,6 +123,17 @@ int res_held(const ResShape& s) {
     return 0;
 }
 
+ResShape res_pick(const std::vector<ResShape>& shapes, int ng) {
+    ResShape best;
+    const int want = std::max(1, std::min(kMaxCluster, 144 / std::max(1, ng)));
+    for (const ResShape& s : shapes) {
+        const bool few = s.cs <= want, best_few = best.cpl && best.cs <= want;
+        const bool better = few != best_few ? few : few ? s.cs > best.cs : s.cs < best.cs;
+        if (best.cpl == 0 || better) best = s;
+    }
+    return best;
+}
+
 void res_receivers(const std::vector<int32_t>& rcv, int nx, int ny, std::vector<int32_t>& chan,
                    std::vector<int32_t>& cell, std::vector<int32_t>& rowstart) {
     chan.clear();

@@ -186,7 +186,6 @@ struct tomo_ctx {
         if (batch_exec) cudaGraphExecDestroy(batch_exec);
         for (void* p : allocs) cudaFree(p);
         if (err_host) cudaFreeHost(err_host);
-        if (pin) cudaFreeHost(pin);
         if (evj) cudaEventDestroy(evj);
         if (ev0) cudaEventDestroy(ev0);
         if (ev1) cudaEventDestroy(ev1);
@@ -814,8 +813,10 @@ tomo_status create_buffers(tomo_ctx* c) {
     }
     c->strip = strip_supported(d, g.cfg.profile) && !std::getenv("TOMO_NO_STRIP");
     // the tile kernels' wait time-out word, written by the device, read by sync_check
-    CU(c, cudaHostAlloc((void**)&c->err_host, sizeof(unsigned int), cudaHostAllocMapped));
+    // (and, 64 bytes on, the results a call reads back: pin)
+    CU(c, cudaHostAlloc((void**)&c->err_host, 128, cudaHostAllocMapped));
     *c->err_host = 0u;
+    c->pin = reinterpret_cast<double*>(c->err_host + 16);
     CU(c, cudaHostGetDevicePointer((void**)&c->err_dev, c->err_host, 0));
     if (const char* e = std::getenv("TOMO_WAIT_LIMIT_NS")) c->wait_ns = std::strtoull(e, nullptr, 10);
     if (const char* e = std::getenv("TOMO_TEST_UNDELIVERED_TX")) c->test_tx = (uint32_t)std::strtoul(e, nullptr, 10);
@@ -1254,9 +1255,10 @@ tomo_status tune_resident(tomo_ctx* c) {
             if (hit) return TOMO_OK;
         }
     const bool tlog = std::getenv("TOMO_TUNE_LOG") != nullptr;
-    const int T = std::min(std::min(c->K, g.nt - 2), 48);
     for (int which = 0; which < (c->P > 1 ? 2 : 1); ++which) {
         const int ng = which == 0 ? 1 : c->P;
+        // long enough that a launch's set-up does not decide, where a step is short
+        const int T = std::min(std::min(c->K, g.nt - 2), (double)ng * g.N < 1e6 ? 160 : 48);
         float best = 1e30f;
         for (const ResShape& s : cands) {
             if (res_held(s) < 1) continue;
@@ -1500,24 +1502,38 @@ tomo_status apply_dir(tomo_ctx* c, const tomo_schedule* s, double scale) {
     return TOMO_OK;
 }
 
-// Sum of the residual partials of all groups -> host.
-tomo_status residual_norm(tomo_ctx* c, double* out) {
+// Sum of the residual partials of all groups into pinned memory (pin[0]); valid after a sync.
+tomo_status enqueue_residual(tomo_ctx* c) {
     const Geometry& g = c->geo;
     launch_sum_parts(c->rpart, 1, g.G * g.nt, c->sums, c->st);
     ++c->launches;
-    CU(c, cudaMemcpyAsync(out, c->sums, sizeof(double), cudaMemcpyDeviceToHost, c->st));
+    CU(c, cudaMemcpyAsync(c->pin, c->sums, sizeof(double), cudaMemcpyDeviceToHost, c->st));
     return TOMO_OK;
 }
 
-tomo_status epsilon(tomo_ctx* c, double* out) {
+// The image-error sums of c->f against c->ftrue into pinned memory (pin[1], pin[2]).
+tomo_status enqueue_epsilon(tomo_ctx* c) {
     const int nb = reduce_blocks();
     launch_eps_parts(c->f, c->ftrue, c->geo.N, c->part, nb, c->st);
     launch_sum_parts(c->part, 2, nb, c->sums + 2, c->st);
     c->launches += 2;
-    double ab[2];
-    CU(c, cudaMemcpyAsync(ab, c->sums + 2, sizeof ab, cudaMemcpyDeviceToHost, c->st));
+    CU(c, cudaMemcpyAsync(c->pin + 1, c->sums + 2, 2 * sizeof(double), cudaMemcpyDeviceToHost, c->st));
+    return TOMO_OK;
+}
+double pinned_epsilon(const tomo_ctx* c) { return 100.0 * std::sqrt(c->pin[1]) / std::sqrt(c->pin[2]); }
+
+// Sum of the residual partials of all groups -> host.
+tomo_status residual_norm(tomo_ctx* c, double* out) {
+    TRY(enqueue_residual(c));
     TRY(sync_check(c));
-    *out = 100.0 * std::sqrt(ab[0]) / std::sqrt(ab[1]);
+    *out = c->pin[0];
+    return TOMO_OK;
+}
+
+tomo_status epsilon(tomo_ctx* c, double* out) {
+    TRY(enqueue_epsilon(c));
+    TRY(sync_check(c));
+    *out = pinned_epsilon(c);
     return TOMO_OK;
 }
 
@@ -1602,17 +1618,9 @@ tomo_status enqueue_iteration(tomo_ctx* c, int method, const tomo_schedule* sch,
         LayoutScope layout(c, pass_layout(c, MODE_GRAD, ng));
         c->launches += record_pass(c, MODE_GRAD, g0, ng);
     }
-    launch_sum_parts(c->rpart, 1, g.G * g.nt, c->sums, c->st);
-    ++c->launches;
-    CU(c, cudaMemcpyAsync(c->pin, c->sums, sizeof(double), cudaMemcpyDeviceToHost, c->st));
+    TRY(enqueue_residual(c));
     TRY(update_core(c, method, sch, s));
-    if (d_ft) {
-        const int nb = reduce_blocks();
-        launch_eps_parts(c->f, c->ftrue, N, c->part, nb, c->st);
-        launch_sum_parts(c->part, 2, nb, c->sums + 2, c->st);
-        c->launches += 2;
-        CU(c, cudaMemcpyAsync(c->pin + 1, c->sums + 2, 2 * sizeof(double), cudaMemcpyDeviceToHost, c->st));
-    }
+    if (d_ft) TRY(enqueue_epsilon(c));
     CU(c, cudaMemcpyAsync(d_f, c->f, sizeof(float) * N, cudaMemcpyDeviceToDevice, c->st));
     *kernels = c->launches - l0;
     return TOMO_OK;
@@ -1634,7 +1642,6 @@ tomo_status record_batch_graph(tomo_ctx** ctxs, int n, int method, const tomo_sc
     for (int i = 0; i < n; ++i) {
         tomo_ctx* c = ctxs[i];
         if (!c->evj) CU(c, cudaEventCreateWithFlags(&c->evj, cudaEventDisableTiming));
-        if (!c->pin) CU(c, cudaHostAlloc((void**)&c->pin, 4 * sizeof(double), cudaHostAllocDefault));
     }
     cudaEvent_t fork = nullptr;
     CU(lead, cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
@@ -1759,10 +1766,8 @@ tomo_status iterate_core(tomo_ctx* c, int method, const tomo_schedule* sch, int 
     const double sc = g.corr_scale;
     const int64_t launches0 = c->launches;
     CU(c, cudaEventRecord(c->ev0, c->st));
-    double r2 = 0.0;
     if (method == TOMO_ART) {
         // art-mimo.cu:688-736: each group sees the field updated by the previous one.
-        double acc = 0.0;
         TRY(next_noise_draw(c));
         for (int gg = 0; gg < G; ++gg) {
             launch_coef(g.cfg.profile, c->f, c->coef, c->rcoef, N, g.cfg.courant, c->st);
@@ -1771,20 +1776,19 @@ tomo_status iterate_core(tomo_ctx* c, int method, const tomo_schedule* sch, int 
             c->launches += 2;
             TRY(apply_dir(c, sch, s));
         }
-        TRY(residual_norm(c, &acc));
-        TRY(sync_check(c));
-        r2 = acc;
+        TRY(enqueue_residual(c));
     } else {
         TRY(gradient_all(c));
-        TRY(residual_norm(c, &r2));
+        TRY(enqueue_residual(c));
         TRY(update_core(c, method, sch, s));
     }
     CU(c, cudaEventRecord(c->ev1, c->st));
-    double eps = std::numeric_limits<double>::quiet_NaN();
-    if (have_true) TRY(epsilon(c, &eps));
+    // one synchronisation per iteration: both results come back through pinned memory
+    if (have_true) TRY(enqueue_epsilon(c));
     TRY(sync_check(c));
     CU(c, cudaGetLastError());
-    fill_stats(c, stats, eps, r2, s, (double)G, launches0);
+    fill_stats(c, stats, have_true ? pinned_epsilon(c) : std::numeric_limits<double>::quiet_NaN(), c->pin[0], s, (double)G,
+               launches0);
     return TOMO_OK;
 }
 

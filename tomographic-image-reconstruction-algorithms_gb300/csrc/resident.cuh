@@ -394,19 +394,21 @@ __global__ void __launch_bounds__(MAXT, 1) k_res_fwd(DevGeo g, ResFwd a) {
             F::load(ua[r], a.in1 + gl * a.instride + (int64_t)j * ROW, lane);
         }
     }
-    // this thread's receiver (the block's receivers are consecutive in row order)
+    // this thread's receiver (the block's receivers are consecutive in row order, dealt out from the second
+    // warp on: the first and the last have the links to attend to)
     const int n0 = a.gout ? a.rowstart[min(jb, ny)] : 0, n1 = a.gout ? a.rowstart[min(jb + RB, ny)] : 0;
     const bool noisy = a.gmeas && g.noise_key;
     const uint64_t key = noisy ? *g.noise_key : 0;
     const int64_t rbase = (int64_t)gl * g.nt * g.nch;
     int roff = 0, rch = 0;
-    const bool rec = n0 + (int)threadIdx.x < n1, rec_more = n0 + (int)blockDim.x < n1;
+    const int ri = 32 * ((w + W - 1) % W) + lane;
+    const bool rec = n0 + ri < n1, rec_more = n0 + (int)blockDim.x < n1;
     if (rec) {
-        const int q = a.rcell[n0 + threadIdx.x], j = q / nx;
+        const int q = a.rcell[n0 + ri], j = q / nx;
         roff = (j - jb) * 2 * ROW + F::col(q - j * nx);
-        rch = a.rchan[n0 + threadIdx.x];
+        rch = a.rchan[n0 + ri];
     }
-    const bool rec_warp = n0 + 32 * w < n1, meas = rec && a.gmeas;
+    const bool rec_warp = n0 + ri - lane < n1, meas = rec && a.gmeas;
     float* op = rec ? a.gout + rbase + (int64_t)(a.k0 + 1) * g.nch + rch : nullptr;         // slice k0 + 1
     const float* mp = meas ? a.gmeas + rbase + (int64_t)(a.k0 + 1) * g.nch + rch : nullptr;
     const float* const pub0 = sm.xch + roff;
@@ -439,7 +441,7 @@ __global__ void __launch_bounds__(MAXT, 1) k_res_fwd(DevGeo g, ResFwd a) {
             op += g.nch;
         }
         if (rec_more) {
-            for (int n = n0 + threadIdx.x + blockDim.x; n < n1; n += blockDim.x) {
+            for (int n = n0 + ri + blockDim.x; n < n1; n += blockDim.x) {
                 const int q = a.rcell[n], j = q / nx, ch = a.rchan[n];
                 const int64_t o = rbase + (int64_t)m * g.nch + ch;
                 put(sm.xch[((j - jb) * 2 + P) * ROW + F::col(q - j * nx)], a.gmeas ? a.gmeas[o] : 0.f, a.gout + o, m, ch);
@@ -671,8 +673,9 @@ __global__ void __launch_bounds__(MAXT, 1) k_res_adj(DevGeo g, ResAdj a) {
     // more); step t's residuals lie in val[t & 1], staged a step before from a register loaded two
     // steps before that
     const float* const rr = a.rr + gl * a.rrstride;
-    const bool stg = (int)threadIdx.x < nrec, stg_more = (int)blockDim.x < nrec;
-    const float* rp = stg ? rr + (int64_t)a.kz0 * g.nch + a.rchan[n0 + threadIdx.x] : nullptr;
+    const int ri = 32 * ((w + W - 1) % W) + lane;
+    const bool stg = ri < nrec, stg_more = (int)blockDim.x < nrec;
+    const float* rp = stg ? rr + (int64_t)a.kz0 * g.nch + a.rchan[n0 + ri] : nullptr;
     int rleft = stg ? T : 0;
     auto next_res = [&](float& v) {
         if (rleft > 0) {
@@ -683,9 +686,9 @@ __global__ void __launch_bounds__(MAXT, 1) k_res_adj(DevGeo g, ResAdj a) {
     };
     auto stage = [&](int t, auto pc, float v) {
         constexpr int P = decltype(pc)::value;
-        if (stg) sm.val[P * nrec + threadIdx.x] = v;
+        if (stg) sm.val[P * nrec + ri] = v;
         if (stg_more && t <= T)
-            for (int n = threadIdx.x + blockDim.x; n < nrec; n += blockDim.x)
+            for (int n = ri + blockDim.x; n < nrec; n += blockDim.x)
                 sm.val[P * nrec + n] = rr[(int64_t)(a.kz0 - t + 1) * g.nch + a.rchan[n0 + n]];
     };
     using P0 = std::integral_constant<int, 0>;

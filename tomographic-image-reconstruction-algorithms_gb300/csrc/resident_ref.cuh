@@ -163,12 +163,13 @@ __global__ void __launch_bounds__(MAXT, 1) k_ref_fwd(DevGeo g, ResFwd a) {
         return (a.rowslot[j] - rank * W * RPW) * 2 * ROW + F::col(q - j * nx);
     };
     int roff = 0, rch = 0;
-    const bool rec = n0 + (int)threadIdx.x < n1, rec_more = n0 + (int)blockDim.x < n1;
+    const int ri = 32 * ((w + W - 1) % W) + lane;
+    const bool rec = n0 + ri < n1, rec_more = n0 + (int)blockDim.x < n1;
     if (rec) {
-        roff = rec_off(n0 + threadIdx.x);
-        rch = a.rchan[n0 + threadIdx.x];
+        roff = rec_off(n0 + ri);
+        rch = a.rchan[n0 + ri];
     }
-    const bool rec_warp = n0 + 32 * w < n1, meas = rec && a.gmeas;
+    const bool rec_warp = n0 + ri - lane < n1, meas = rec && a.gmeas;
     float* op = rec ? a.gout + rbase + (int64_t)(a.k0 + 1) * g.nch + rch : nullptr;         // slice k0 + 1
     const float* mp = meas ? a.gmeas + rbase + (int64_t)(a.k0 + 1) * g.nch + rch : nullptr;
     const float* const pub0 = sm.xch + roff;
@@ -200,7 +201,7 @@ __global__ void __launch_bounds__(MAXT, 1) k_ref_fwd(DevGeo g, ResFwd a) {
             op += g.nch;
         }
         if (rec_more) {
-            for (int n = n0 + threadIdx.x + blockDim.x; n < n1; n += blockDim.x) {
+            for (int n = n0 + ri + blockDim.x; n < n1; n += blockDim.x) {
                 const int ch = a.rchan[n];
                 const int64_t o = rbase + (int64_t)m * g.nch + ch;
                 put(sm.xch[rec_off(n) + P * ROW], a.gmeas ? a.gmeas[o] : 0.f, a.gout + o, m, ch);
@@ -556,8 +557,9 @@ __global__ void __launch_bounds__(MAXT, 1) k_ref_adj(DevGeo g, ResAdj a) {
         rb[r] = j == lo || j == hi ? f + max(0, CPL * lane - (lo + 1)) : f;   // columns lo+1 .. hi-1; lo and hi
     }
     const float* const rr = a.rr + gl * a.rrstride;
-    const bool stg = (int)threadIdx.x < nrec, stg_more = (int)blockDim.x < nrec;
-    const float* rp = stg ? rr + (int64_t)a.kz0 * g.nch + a.rchan[n0 + threadIdx.x] : nullptr;
+    const int ri = 32 * ((w + W - 1) % W) + lane;
+    const bool stg = ri < nrec, stg_more = (int)blockDim.x < nrec;
+    const float* rp = stg ? rr + (int64_t)a.kz0 * g.nch + a.rchan[n0 + ri] : nullptr;
     int rleft = stg ? T : 0;
     auto next_res = [&](float& v) {
         if (rleft > 0) {
@@ -569,9 +571,9 @@ __global__ void __launch_bounds__(MAXT, 1) k_ref_adj(DevGeo g, ResAdj a) {
     auto inject = [](float v) { return xm(xm(v, kRefH), 1000.f); };   // (rr H) 1000
     auto stage = [&](int t, auto pc, float v) {
         constexpr int P = decltype(pc)::value;
-        if (stg) sm.val[P * nrec + threadIdx.x] = inject(v);
+        if (stg) sm.val[P * nrec + ri] = inject(v);
         if (stg_more && t <= T)
-            for (int n = threadIdx.x + blockDim.x; n < nrec; n += blockDim.x)
+            for (int n = ri + blockDim.x; n < nrec; n += blockDim.x)
                 sm.val[P * nrec + n] = inject(rr[(int64_t)(a.kz0 - t + 1) * g.nch + a.rchan[n0 + n]]);
     };
     using P0 = std::integral_constant<int, 0>;

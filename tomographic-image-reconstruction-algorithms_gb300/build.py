@@ -24,7 +24,7 @@ NVCC = os.environ.get("NVCC", "nvcc")
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 COMMON = ["-O3", "-std=c++17", "-lineinfo", "-I" + INCLUDE, "-I" + CSRC]
 
-LIB_SOURCES = ["kernels.cu", "strip.cu", "tile.cu", "resident.cu", "resident_a.cu", "resident_b.cu",
+LIB_SOURCES = ["kernels.cu", "strip.cu", "tile.cu", "stream.cu", "resident.cu", "resident_a.cu", "resident_b.cu",
                "resident_c.cu", "resident_d.cu", "resident_e.cu", "resident_f.cu", "engine.cu", "geometry.cpp", "noalloc.cu", "cnn.cu", "net.cu"]
 # driver name -> -D selector of cli/tomo_cli.cpp
 DRIVERS = {

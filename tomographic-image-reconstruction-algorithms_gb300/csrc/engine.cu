@@ -91,6 +91,11 @@ struct tomo_ctx {
     int32_t *warps = nullptr, *rowslot = nullptr;   // reference profile: rows of each warp, slot of each row
     std::vector<ResShape> res_cands;   // every shape that holds a group (tune_resident times them)
     bool res_tuned = false;
+    // several steps per launch on grids that do not fit on chip (stream.cu): possible, and chosen for passes
+    // of P groups and of one; framed slices of pitch px
+    bool stream_ok = false, stream = false, stream1 = false;
+    int px = 0;
+    float *ust = nullptr, *corrp = nullptr, *coefp = nullptr, *dmapp = nullptr;
     // learned iteration (allocated on first use)
     float *illum = nullptr, *feat = nullptr, *fsave = nullptr, *dnet = nullptr, *dsave = nullptr;
     unsigned int *illum_max = nullptr, *maxsave = nullptr;
@@ -99,6 +104,7 @@ struct tomo_ctx {
     int learned_backtrack = 0;   // retries of a rejected proposal at half the scale (tomo_run_learned)
     int learned_resume = 0;      // plain steps after which paused proposals resume (0: never)
     static constexpr int ZR = 4; // adjoint ring slots
+    static constexpr int UR = 4; // wavefield ring slots of the streamed sweeps
     TileMaps tmaps;              // TMA maps of hist, z, coef, dmap, rid (tile kernels)
     TileMaps tmaps_ck;           // the same with the slice maps over the checkpoint buffer (pass_layout)
     unsigned int* err_host = nullptr;   // tile kernels' wait time-out word (mapped pinned memory)
@@ -631,7 +637,9 @@ double plan_bytes_per_group(const tomo_ctx* c, bool full, int K) {
     const int64_t nt = g.nt;
     const int64_t slots = full ? nt : (int64_t)K + 1;
     const int64_t chunks = full ? 0 : (nt - 2 + K - 1) / K;
-    return 4.0 * ((double)(slots + tomo_ctx::ZR + 2 * chunks) * c->NS + (double)nt * g.nch);
+    // the streamed sweeps' wavefield ring and framed correlation
+    const int64_t more = c->stream_ok ? tomo_ctx::UR + 1 : 0;
+    return 4.0 * ((double)(slots + tomo_ctx::ZR + 2 * chunks + more) * c->NS + (double)nt * g.nch);
 }
 
 // The plan with the most groups per pass that fits c->plan_budget (or the configured P).
@@ -673,7 +681,16 @@ void choose_resident(tomo_ctx* c) {
         c->res_cands = res_shapes(g.nx, g.ny, c->h_rowstart);
     }
     while (!c->res_cands.empty() && res_held(c->res_cands.back()) < 1) c->res_cands.pop_back();
-    if (c->res_cands.empty()) return;
+    const char* s = std::getenv("TOMO_STREAM");   // 1: streamed whatever the size (tests), 0: not streamed
+    if (!g.ref && s && *s == '1') c->res_cands.clear();
+    if (c->res_cands.empty()) {
+        c->stream_ok = !g.ref && !(s && *s == '0');
+        if (c->stream_ok) {
+            c->px = stream_pitch(g.nx);
+            c->NS = stream_slice(g.nx, g.ny);
+        }
+        return;
+    }
     c->res = c->res1 = c->res_cands.back();   // tune_resident picks among them
     c->NS = res_slice(c->res, g.ny);
 }
@@ -694,13 +711,20 @@ tomo_status make_plan(tomo_ctx* c) {
     if (g.cfg.mem_limit_mb > 0) cap = std::min(cap, (double)g.cfg.mem_limit_mb * (1 << 20));
     c->plan_budget = cap - (double)fixed;
     const int K = g.cfg.ckpt_interval;
-    Plan p{};
-    if (K > 0) {
-        if (K < nt - 2 && K < 2) return c->fail(TOMO_ERR_ARG, "ckpt_interval must be >= 2");
-        p = plan_of(c, K >= nt - 2, K);
-    } else {
-        p = plan_of(c, true, 0);
-        if (p.P < (g.cfg.groups_per_pass > 0 ? std::min<int64_t>(g.cfg.groups_per_pass, G) : G)) p = plan_of(c, false, std::max(2, (int)std::ceil(std::sqrt(2.0 * (double)(nt - 2)))));
+    if (K > 0 && K < nt - 2 && K < 2) return c->fail(TOMO_ERR_ARG, "ckpt_interval must be >= 2");
+    auto choose = [&] {
+        if (K > 0) return plan_of(c, K >= nt - 2, K);
+        const Plan p = plan_of(c, true, 0);
+        if (p.P >= (g.cfg.groups_per_pass > 0 ? std::min<int64_t>(g.cfg.groups_per_pass, G) : G)) return p;
+        return plan_of(c, false, std::max(2, (int)std::ceil(std::sqrt(2.0 * (double)(nt - 2)))));
+    };
+    Plan p = choose();
+    if (p.P < 1 && c->NS != g.N) {   // the padded slices do not fit: the per-step kernels' may
+        c->res = c->res1 = ResShape{};
+        c->res_cands.clear();
+        c->stream_ok = false;
+        c->NS = g.N;
+        p = choose();
     }
     if (p.P < 1)
         return c->fail(TOMO_ERR_OOM, "plan needs %.2f GB for one group per pass, %.2f GB available",
@@ -718,6 +742,11 @@ tomo_status alloc_plan_buffers(tomo_ctx* c) {
     TRY(c->alloc(&c->z, P * tomo_ctx::ZR * N, "adjoint slots"));
     if (!c->full) TRY(c->alloc(&c->ckpt, P * c->nchunk * 2 * N, "checkpoints"));
     TRY(c->alloc(&c->rr, P * g.nt * g.nch, "residual records"));
+    if (c->stream_ok) {
+        TRY(c->alloc(&c->ust, P * tomo_ctx::UR * N, "wavefield ring"));
+        TRY(c->alloc(&c->corrp, P * N, "framed correlation"));
+        CU(c, cudaMemsetAsync(c->ust, 0, sizeof(float) * (size_t)(P * tomo_ctx::UR * N), c->st));
+    }
     CU(c, cudaMemsetAsync(c->hist, 0, sizeof(float) * (size_t)P * c->S * N, c->st));
     CU(c, cudaMemsetAsync(c->z, 0, sizeof(float) * (size_t)P * tomo_ctx::ZR * N, c->st));
     CU(c, cudaMemsetAsync(c->rr, 0, sizeof(float) * (size_t)(P * g.nt * g.nch), c->st));
@@ -810,6 +839,11 @@ tomo_status create_buffers(tomo_ctx* c) {
         CU(c, cudaMemcpyAsync(c->dmap, dm.data(), sizeof(float) * N, cudaMemcpyHostToDevice, c->st));
         TRY(sync_check(c));   // `dm` is local
         d.dmap = c->dmap;
+    }
+    if (c->stream_ok) {
+        TRY(c->alloc(&c->coefp, c->NS, "framed coefficient"));
+        TRY(c->alloc(&c->dmapp, c->NS, "framed sponge map"));
+        launch_frame(c->dmapp, c->dmap, g.nx, g.ny, c->st);
     }
     c->strip = strip_supported(d, g.cfg.profile) && !std::getenv("TOMO_NO_STRIP");
     // the tile kernels' wait time-out word, written by the device, read by sync_check
@@ -935,10 +969,171 @@ int64_t record_resident_pass(tomo_ctx* c, int mode, int g0, int ng) {
     return n;
 }
 
+// Steps of the next streamed launch when L remain: the last launch of a segment advances two or more
+// steps where the segment has them, so both slices of its end state come from one launch.
+int stream_steps(int L) { return L >= 6 || L == 4 ? 4 : L % 2 ? 1 : 2; }
+
+// The wavefield state of a streamed sweep: slices k-1 and k, each with its group stride.
+struct StreamState {
+    float *p0, *p1;
+    int64_t s0, s1;
+};
+
+// Forward steps of a streamed pass from slice k0 (state st) to slice k0 + T, L(q) of q >= qlo kept when
+// keep, the end state written to end0, end1 (null: the ring).  Returns the launches.
+int64_t stream_forward(tomo_ctx* c, StreamState& st, int k0, int T, int g0, int ng, bool keep, int qlo, float* gout, float* end0,
+                       float* end1, int64_t endstride) {
+    int64_t n = 0;
+    const int64_t NS = c->NS, us = tomo_ctx::UR * NS;
+    while (T > 0) {
+        StreamFwd a{};
+        a.T = stream_steps(T);
+        a.coef = c->coefp;
+        a.dmap = c->dmapp;
+        a.in0 = st.p0;
+        a.in1 = st.p1;
+        a.in0stride = st.s0;
+        a.in1stride = st.s1;
+        if (T == a.T && end0) {
+            a.out0 = end0;
+            a.out1 = end1;
+            a.outstride = endstride;
+        } else {   // two ring slots the inputs are not in
+            float* free[2] = {nullptr, nullptr};
+            for (int k = 0, f = 0; k < tomo_ctx::UR && f < 2; ++k) {
+                float* s = c->ust + k * NS;
+                if (s != st.p0 && s != st.p1) free[f++] = s;
+            }
+            a.out0 = free[0];
+            a.out1 = free[1];
+            a.outstride = us;
+        }
+        a.hist = keep ? c->hist : nullptr;
+        a.hstride = (int64_t)c->S * NS;
+        a.ns = NS;
+        a.qlo = qlo;
+        a.k0 = k0;
+        a.g0 = g0;
+        a.ng = ng;
+        a.px = c->px;
+        a.gout = gout;
+        a.rec = StreamRec{c->rchan, c->rcell, c->rowstart};
+        launch_stream_fwd(c->dg, a, c->st);
+        ++n;
+        if (a.T == 1) st = StreamState{st.p1, a.out1, st.s1, a.outstride};
+        else st = StreamState{a.out0, a.out1, a.outstride, a.outstride};
+        k0 += a.T;
+        T -= a.T;
+    }
+    return n;
+}
+
+// Adjoint steps of a streamed pass: z(kz0) .. z(kz0-T+1) from the state (p0 = z(kz0+2), p1 = z(kz0+1))
+// in the adjoint ring.
+int64_t stream_adjoint(tomo_ctx* c, StreamState& st, int kz0, int T, int g0, int ng, int qlo) {
+    int64_t n = 0;
+    const int64_t NS = c->NS;
+    while (T > 0) {
+        StreamAdj a{};
+        a.T = T >= 4 ? 4 : T >= 2 ? 2 : 1;
+        a.coef = c->coefp;
+        a.dmap = c->dmapp;
+        a.in0 = st.p0;
+        a.in1 = st.p1;
+        float* free[2] = {nullptr, nullptr};
+        for (int k = 0, f = 0; k < tomo_ctx::ZR && f < 2; ++k) {
+            float* s = c->z + k * NS;
+            if (s != st.p0 && s != st.p1) free[f++] = s;
+        }
+        a.out0 = free[0];
+        a.out1 = free[1];
+        a.instride = tomo_ctx::ZR * NS;
+        a.hist = c->hist;
+        a.hstride = (int64_t)c->S * NS;
+        a.ns = NS;
+        a.qlo = qlo;
+        a.rr = c->rr;
+        a.rrstride = c->recs_per_group();
+        a.corr = c->corrp;
+        a.cstride = NS;
+        a.kz0 = kz0;
+        a.ng = ng;
+        a.px = c->px;
+        a.rec = StreamRec{c->rchan, c->rcell, c->rowstart};
+        launch_stream_adj(c->dg, a, c->st);
+        ++n;
+        if (a.T == 1) st.p0 = st.p1;
+        else st.p0 = a.out0;
+        st.p1 = a.out1;
+        kz0 -= a.T;
+        T -= a.T;
+    }
+    return n;
+}
+
+// A pass by the streamed sweeps (stream.cu).
+int64_t record_stream_pass(tomo_ctx* c, int mode, int g0, int ng) {
+    const Geometry& g = c->geo;
+    const int nt = g.nt, K = c->K;
+    const int64_t NS = c->NS, us = tomo_ctx::UR * NS, zs = tomo_ctx::ZR * NS, rpg = c->recs_per_group(),
+                  cks = (int64_t)c->nchunk * 2 * NS;
+    const bool grad = mode == MODE_GRAD, resid = grad || mode == MODE_RESID;
+    int64_t n = 0;
+    launch_frame(c->coefp, c->coef, g.nx, g.ny, c->st);
+    ++n;
+    if (grad && c->nchunk > 1) {
+        launch_zero_frame(c->ckpt, (int64_t)ng * c->nchunk * 2, g.nx, g.ny, c->st);
+        ++n;
+    }
+    auto zero_state = [&] {
+        launch_zero_slots(c->ust, ng, us, 0, NS, NS, c->st);
+        ++n;
+        return StreamState{c->ust, c->ust + NS, us, us};
+    };
+    float* const gout = resid ? c->rr : c->rec + (int64_t)g0 * rpg;
+    StreamState st = zero_state();
+    const int last = grad ? c->nchunk - 1 : 0;
+    for (int ch = 0; ch <= last; ++ch) {   // segments of the forward sweep, each up to the next chunk's state
+        const int qa = 1 + ch * K, end = ch == last ? nt - 1 : qa + K;
+        float* const ck = ch < last ? c->ckpt + (int64_t)(ch + 1) * 2 * NS : nullptr;
+        n += stream_forward(c, st, qa, end - qa, g0, ng, grad && ch == last, qa, gout, ck, ck ? ck + NS : nullptr, cks);
+    }
+    if (mode == MODE_FWD) {
+        launch_unframe(c->hist + c->slot(nt - 1), (int64_t)c->S * g.N, st.p1, st.s1, g.nx, g.ny, ng, c->st);
+        ++n;
+    }
+    if (resid) {
+        launch_resid_meas(c->dg, c->rr, c->meas + (int64_t)g0 * rpg, g0, ng, c->rpart + (int64_t)g0 * nt, c->st);
+        ++n;
+    }
+    if (!grad) return n;
+    cudaMemsetAsync(c->corrp, 0, sizeof(float) * NS * ng, c->st);
+    cudaMemsetAsync(c->z, 0, sizeof(float) * zs * ng, c->st);
+    StreamState zst{c->z, c->z + NS, zs, zs};
+    for (int ch = last; ch >= 0; --ch) {
+        const int qa = 1 + ch * K, qb = std::min(qa + K - 1, nt - 2), T = qb - qa + 1;
+        if (ch < last) {
+            StreamState r;
+            if (ch > 0) {
+                float* const ck = c->ckpt + (int64_t)ch * 2 * NS;
+                r = StreamState{ck, ck + NS, cks, cks};
+            } else {
+                r = zero_state();
+            }
+            n += stream_forward(c, r, qa, T, g0, ng, true, qa, nullptr, nullptr, nullptr, 0);
+        }
+        n += stream_adjoint(c, zst, qb + 1, T, g0, ng, qa);
+    }
+    launch_unframe(c->corr + (int64_t)g0 * g.N, g.N, c->corrp, NS, g.nx, g.ny, ng, c->st);
+    ++n;
+    return n;
+}
+
 // Records the launch sequence of one pass (groups g0 .. g0+ng-1) on the stream.
 // Kernel nodes the recorded pass contains (each launch_* call below is one kernel).
 int64_t record_pass(tomo_ctx* c, int mode, int g0, int ng) {
     if (c->res.cpl && mode != MODE_ILLUM) return record_resident_pass(c, mode, g0, ng);
+    if ((ng == 1 ? c->stream1 : c->stream) && mode != MODE_ILLUM) return record_stream_pass(c, mode, g0, ng);
     int64_t n = 0;
     // multi-step tile kernels: the choice made for passes of one group when the pass has one
     const bool tile_fwd = ng == 1 ? c->tile_fwd1 : c->tile_fwd;
@@ -1168,7 +1363,7 @@ PassLayout pass_layout(const tomo_ctx* c, int mode, int ng) {
     if (L >= nt) return PassLayout{nt, nt - 2, 1, true, false};
     // a pass with full history needs no checkpoints: the checkpoint buffer (P nchunk 2 slices)
     // holds the history when the slot buffer does not (tile kernels need its maps)
-    const bool ck_maps = c->res.cpl || !(ng == 1 ? c->tile_fwd1 || c->tile_adj1 : c->tile_fwd || c->tile_adj) || c->tmaps_ck.ok;
+    const bool ck_maps = c->res.cpl || (ng == 1 ? c->stream1 : c->stream) || !(ng == 1 ? c->tile_fwd1 || c->tile_adj1 : c->tile_fwd || c->tile_adj) || c->tmaps_ck.ok;
     if ((int64_t)c->P * c->nchunk * 2 / ng >= nt && ck_maps) return PassLayout{nt, nt - 2, 1, true, true};
     int nchunk = (int)((nt - 2 + L - 2) / (L - 1));
     int K = (nt - 1 + nchunk - 1) / nchunk;
@@ -1298,12 +1493,118 @@ tomo_status tune_resident(tomo_ctx* c) {
     return TOMO_OK;
 }
 
+// `steps` forward (which 0) or adjoint steps of the first ng groups with the kernels chosen for such
+// passes, from slice k0 (adjoint: down to it); keep: resident and streamed forward steps store the history.
+void enqueue_steps(tomo_ctx* c, int which, int k0, int steps, int ng, bool keep) {
+    const Geometry& g = c->geo;
+    for (int t = 0; t < steps;) {
+        if (c->res.cpl) {   // a chunk of steps per launch, with the history traffic of a sweep
+            const ResShape& s = ng == 1 ? c->res1 : c->res;
+            const int T = std::min(steps - t, c->K);
+            if (which == 0) {
+                ResFwd f = res_fwd_args(c, s, k0, T, 0, ng);
+                f.hist = keep ? c->hist : nullptr;
+                f.qlo = k0;
+                launch_res_fwd(s, c->dg, f, c->st);
+            } else {
+                ResAdj a = res_adj_args(c, s, g.ref ? k0 + T - 1 : k0 + T, T, 0, ng);
+                a.qlo = k0;
+                a.first = true;
+                launch_res_adj(s, c->dg, a, c->st);
+            }
+            t += T;
+        } else if (ng == 1 ? c->stream1 : c->stream) {
+            const int T = std::min(steps - t, c->K);
+            StreamState u{c->ust, c->ust + c->NS, tomo_ctx::UR * c->NS, tomo_ctx::UR * c->NS};
+            StreamState z{c->z, c->z + c->NS, tomo_ctx::ZR * c->NS, tomo_ctx::ZR * c->NS};
+            if (which == 0) stream_forward(c, u, k0, T, 0, ng, keep, k0, nullptr, nullptr, nullptr, 0);
+            else stream_adjoint(c, z, k0 + T, T, 0, ng, k0);
+            t += T;
+        } else if (which == 0 && c->tile_fwd) {
+            const int T = tile_fwd_steps(c, steps - t);
+            launch_fwd_tile(c->dg, c->tmaps, tile_fwd_args(c, k0 + t, T, 0, ng), c->st);
+            t += T;
+        } else if (which == 1 && c->tile_adj) {
+            const int T = tile_adj_steps(steps - t);
+            launch_adj_tile(c->dg, c->tmaps, tile_adj_args(c, k0 + steps - t, T, 0, ng), c->st);
+            t += T;
+        } else if (which == 0 && c->fwd_pair && t + 1 < steps) {
+            launch_fwd2_strip(c->rows_fwd2, c->dg, c->coef, fwd_args(c, k0 + t, 0, ng), fwd_args(c, k0 + t + 1, 0, ng),
+                              false, false, c->st);
+            t += 2;
+        } else if (which == 0) {
+            fwd_launch(c, fwd_args(c, k0 + t, 0, ng));
+            t += 1;
+        } else if (c->adj_pair && t + 1 < steps) {
+            const int q = k0 + steps - 1 - t;
+            launch_adj2_strip(c->rows_adj2, c->dg, c->coef, adj_args(c, q, 0, ng), adj_args(c, q - 1, 0, ng), c->st);
+            t += 2;
+        } else {
+            adj_launch(c, adj_args(c, k0 + steps - 1 - t, 0, ng));
+            t += 1;
+        }
+    }
+}
+
+// Chooses between the streamed sweeps and the per-step (or tile) kernels autotune has picked, for
+// passes of P groups and of one, by timing steps of each: per step a pass costs a forward step
+// (streamed: with the history kept, in the last chunk only), for all chunks but one a recomputed forward
+// step with the history, and an adjoint step.  Sweeps too short for a trial keep the strip kernels where
+// the width allows them (a multiple of 4) and are streamed otherwise.  TOMO_STREAM=1 fixes the choice.
+tomo_status tune_stream(tomo_ctx* c) {
+    if (c->tuned) return TOMO_OK;
+    const char* e = std::getenv("TOMO_STREAM");
+    const int steps = 16, nt = c->geo.nt;
+    if (c->stream_ok && ((!c->strip && nt < 4 * steps) || (e && *e == '1'))) {
+        c->tuned = c->stream = c->stream1 = true;
+        return TOMO_OK;
+    }
+    TRY(autotune(c));
+    if (!c->stream_ok || nt < 4 * steps) return TOMO_OK;
+    const int k0 = nt / 2 - steps;
+    const double again = (double)(c->nchunk - 1) / c->nchunk;
+    auto time_steps = [&](int which, int ng, bool keep, double& ms) -> tomo_status {
+        ms = 1e30;
+        for (int pass = 0; pass < 3; ++pass) {   // the first warms up
+            CU(c, cudaEventRecord(c->ev0, c->st));
+            enqueue_steps(c, which, k0, steps, ng, keep);
+            CU(c, cudaEventRecord(c->ev1, c->st));
+            CU(c, cudaEventSynchronize(c->ev1));
+            CU(c, cudaGetLastError());
+            float t = 0.f;
+            CU(c, cudaEventElapsedTime(&t, c->ev0, c->ev1));
+            if (pass > 0) ms = std::min(ms, (double)t);
+        }
+        return TOMO_OK;
+    };
+    bool better[2] = {false, false};
+    for (int one = 0; one < 2; ++one) {
+        const int ng = one ? 1 : c->P;
+        double f = 0.0, a = 0.0, fn = 0.0, fk = 0.0, b = 0.0;
+        c->stream = c->stream1 = false;
+        TRY(time_steps(0, ng, true, f));
+        TRY(time_steps(1, ng, true, a));
+        c->stream = c->stream1 = true;
+        TRY(time_steps(0, ng, false, fn));
+        TRY(time_steps(0, ng, true, fk));
+        TRY(time_steps(1, ng, true, b));
+        better[one] = again * fn + fk + b < f * (1.0 + again) + a;
+        if (std::getenv("TOMO_TUNE_LOG"))
+            std::fprintf(stderr, "tomo tune: %d groups, us per step: per-step kernels forward %.2f adjoint %.2f, streamed forward "
+                         "%.2f (with history %.2f) adjoint %.2f\n", ng, 1e3 * f / steps, 1e3 * a / steps, 1e3 * fn / steps,
+                         1e3 * fk / steps, 1e3 * b / steps);
+    }
+    c->stream = better[0];
+    c->stream1 = c->P > 1 ? better[1] : better[0];
+    return TOMO_OK;
+}
+
 tomo_status run_pass(tomo_ctx* c, int mode, int g0, int ng) {
     const auto key = std::make_tuple(mode, g0, ng);
     auto it = c->graphs.find(key);
     if (it == c->graphs.end()) {
-        if (!c->res.cpl || mode == MODE_ILLUM) TRY(autotune(c));
-        else TRY(tune_resident(c));
+        if (c->res.cpl) TRY(mode == MODE_ILLUM ? autotune(c) : tune_resident(c));
+        else TRY(tune_stream(c));
         LayoutScope layout(c, pass_layout(c, mode, ng));
         cudaGraph_t graph = nullptr;
         CU(c, cudaStreamBeginCapture(c->st, cudaStreamCaptureModeThreadLocal));
@@ -1379,6 +1680,8 @@ tomo_status apply_plan(tomo_ctx* c, const Plan& p) {
     c->release(&c->z);
     c->release(&c->ckpt);
     c->release(&c->rr);
+    c->release(&c->ust);
+    c->release(&c->corrp);
     set_plan(c, p);
     c->tuned = c->res_tuned = false;
     ++c->gen;
@@ -1713,8 +2016,7 @@ tomo_status iterate_batch_graph(tomo_ctx** ctxs, int n, int method, const tomo_s
         tomo_ctx* c = ctxs[i];
         if (c->res.cpl ? !c->res_tuned : !c->tuned) {
             launch_coef(c->geo.cfg.profile, c->f, c->coef, c->rcoef, c->geo.N, c->geo.cfg.courant, c->st);
-            if (c->res.cpl) TRY(tune_resident(c));
-            else TRY(autotune(c));
+            TRY(c->res.cpl ? tune_resident(c) : tune_stream(c));
         }
     }
     uint64_t sbits = 0;
@@ -2386,52 +2688,12 @@ tomo_status tomo_time_kernel(tomo_ctx* c, int32_t which, int32_t steps, double* 
     steps = std::min(steps, nt - 4);
     const int k0 = std::max(2, (nt - steps) / 2);
     launch_coef(prof, c->f, c->coef, c->rcoef, N, g.cfg.courant, c->st);
-    if (!c->res.cpl) TRY(autotune(c));
-    else TRY(tune_resident(c));
+    TRY(c->res.cpl ? tune_resident(c) : tune_stream(c));
     // the steps are captured into a graph and replayed, as the iterations run them, so the time
     // per step carries the launch gaps of graph replay, not of stream launches
     cudaGraph_t graph = nullptr;
     CU(c, cudaStreamBeginCapture(c->st, cudaStreamCaptureModeThreadLocal));
-    for (int t = 0; t < steps;) {
-        if (c->res.cpl) {   // a chunk of steps per launch, with the history traffic of a sweep
-            const ResShape& s = ng == 1 ? c->res1 : c->res;
-            const int T = std::min(steps - t, c->K);
-            if (which == 0) {
-                ResFwd f = res_fwd_args(c, s, k0, T, 0, ng);
-                f.hist = c->hist;
-                f.qlo = k0;
-                launch_res_fwd(s, c->dg, f, c->st);
-            } else {
-                ResAdj a = res_adj_args(c, s, g.ref ? k0 + T - 1 : k0 + T, T, 0, ng);
-                a.qlo = k0;
-                a.first = true;
-                launch_res_adj(s, c->dg, a, c->st);
-            }
-            t += T;
-        } else if (which == 0 && c->tile_fwd) {
-            const int T = tile_fwd_steps(c, steps - t);
-            launch_fwd_tile(c->dg, c->tmaps, tile_fwd_args(c, k0 + t, T, 0, ng), c->st);
-            t += T;
-        } else if (which == 1 && c->tile_adj) {
-            const int T = tile_adj_steps(steps - t);
-            launch_adj_tile(c->dg, c->tmaps, tile_adj_args(c, k0 + steps - t, T, 0, ng), c->st);
-            t += T;
-        } else if (which == 0 && c->fwd_pair && t + 1 < steps) {
-            launch_fwd2_strip(c->rows_fwd2, c->dg, c->coef, fwd_args(c, k0 + t, 0, ng), fwd_args(c, k0 + t + 1, 0, ng),
-                              false, false, c->st);
-            t += 2;
-        } else if (which == 0) {
-            fwd_launch(c, fwd_args(c, k0 + t, 0, ng));
-            t += 1;
-        } else if (c->adj_pair && t + 1 < steps) {
-            const int q = k0 + steps - 1 - t;
-            launch_adj2_strip(c->rows_adj2, c->dg, c->coef, adj_args(c, q, 0, ng), adj_args(c, q - 1, 0, ng), c->st);
-            t += 2;
-        } else {
-            adj_launch(c, adj_args(c, k0 + steps - 1 - t, 0, ng));
-            t += 1;
-        }
-    }
+    enqueue_steps(c, which, k0, steps, ng, true);
     const cudaError_t ec = cudaStreamEndCapture(c->st, &graph);
     if (ec != cudaSuccess) {
         if (graph) cudaGraphDestroy(graph);

@@ -388,6 +388,51 @@ void res_receivers(const std::vector<int32_t>& rcv, int nx, int ny, std::vector<
                    std::vector<int32_t>& cell, std::vector<int32_t>& rowstart);
 void launch_res_fwd(const ResShape& s, const DevGeo& g, const ResFwd& a, void* stream);
 void launch_res_adj(const ResShape& s, const DevGeo& g, const ResAdj& a, void* stream);
+// ---- several steps per launch on large grids (stream.cu): CFG profile ---------------------------
+// Slices carry a frame of guard cells: cell (x, y) is float (y + STREAM_TOP) px + STREAM_LEFT + x of its
+// ns floats (stream_pitch, stream_slice).
+constexpr int STREAM_TOP = 8, STREAM_BOTTOM = 16, STREAM_LEFT = 8;
+struct StreamRec {
+    const int32_t *rchan, *rcell, *rowstart;   // receivers in row order (cells of the unpadded grid)
+};
+struct StreamFwd {
+    const float *coef, *dmap;       // framed
+    const float *in0, *in1;         // u(k0-1), u(k0)
+    int64_t in0stride, in1stride;
+    float *out0, *out1;             // u(k0+T-1) (T > 1), u(k0+T): not the inputs' slices
+    int64_t outstride;
+    float* hist;                    // L(q), q = k0 .. k0+T-1, to slot q - qlo (null: none)
+    int64_t hstride, ns;
+    int qlo;
+    int k0, T, g0, ng, px;          // T in {1, 2, 4}
+    float* gout;                    // simulated samples of slices k0+1 .. k0+T (null: none)
+    StreamRec rec;
+    int R, bands, strips;           // the launch's cut (set by the launcher)
+};
+struct StreamAdj {
+    const float *coef, *dmap;
+    const float *in0, *in1;         // z(kz0+2), z(kz0+1)
+    float *out0, *out1;             // z(kz0-T+2) (T > 1), z(kz0-T+1): not the inputs' slices
+    int64_t instride;
+    const float* hist;              // L(q) at slot q - qlo; z(m) pairs with L(m-1)
+    int64_t hstride, ns;
+    int qlo;
+    const float* rr;                // residuals of pass-group 0: step m at rr + m * nch
+    int64_t rrstride;
+    float* corr;                    // framed correlation, updated in place
+    int64_t cstride;
+    int kz0, T, ng, px;
+    StreamRec rec;
+    int R, bands, strips;
+};
+int stream_pitch(int nx);
+int64_t stream_slice(int nx, int ny);
+void launch_stream_fwd(const DevGeo& g, const StreamFwd& a, void* stream);
+void launch_stream_adj(const DevGeo& g, const StreamAdj& a, void* stream);
+void launch_resid_meas(const DevGeo& g, float* rr, const float* meas, int g0, int ng, double* part, void* stream);
+void launch_frame(float* dst, const float* src, int nx, int ny, void* stream);
+void launch_unframe(float* dst, int64_t dstride, const float* src, int64_t sstride, int nx, int ny, int planes, void* stream);
+void launch_zero_frame(float* p, int64_t planes, int nx, int ny, void* stream);
 // cuTensorMapEncodeTiled, looked up from the driver once (no link against libcuda); null when
 // the driver has none.
 void* tensor_map_encoder();

@@ -362,7 +362,7 @@ tomo_status tomo_iterate_batch(tomo_ctx** ctxs, int32_t n, int32_t method, const
  * (G*nt*n_channels, the tomo_forward layout) are caller-owned device buffers on
  * the current device; work is enqueued on `stream` (NULL: legacy default) and
  * the records are valid once it completes.  The wavefield scratch lives in a
- * fixed file-scope device array of about 5.1 MiB that each GPU loading the
+ * fixed file-scope device array of about 5.6 MiB that each GPU loading the
  * library holds until exit, so problems are limited to 512*512 cells, 2048
  * record channels and 16384 time steps (and 4096 emitters in the benchmark
  * profile, 2048 groups in the reference profile); larger ones return

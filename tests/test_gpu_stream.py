@@ -103,3 +103,32 @@ def test_least_memory_falls_back(monkeypatch):
         outs += 1
         break
     assert outs == 1
+
+
+@pytest.mark.parametrize("cfg", [
+    ring(nx=512, ny=512, nt=60, ns=16, gs=4),                        # the largest: framed slices fill the array
+    ring(nx=449, ny=451, nt=61, ns=150, gs=50, sponge=0),            # as it comes; one step left over
+    ring(nx=700, ny=371, nt=62, ns=24, gs=8), ring(nx=301, ny=700, nt=63, ns=24, gs=8),
+    ring(nx=250, ny=1000, nt=5, ns=8, gs=8), ring(nx=400, ny=388, nt=4, ns=8, gs=4),
+    ring(nx=9, ny=1030, nt=20, ns=2, gs=1, sponge=2),                # more rows than tables: per-cell kernels
+    ring(nx=13000, ny=20, nt=20, ns=4, gs=1, sponge=2),              # the frame does not fit: per-cell kernels
+], ids=lambda c: f"{c.nx}x{c.ny}")
+def test_allocation_free_forward_streams(cfg, monkeypatch):
+    import ctypes as C
+
+    import torch
+
+    fo = phantom(cfg)
+    monkeypatch.setenv("TOMO_RESIDENT", "0")
+    with tomo.Context(cfg) as ctx:
+        want = ctx.forward(fo)
+    monkeypatch.delenv("TOMO_RESIDENT")
+    d_f = torch.from_numpy(fo).cuda()
+    d_rec = torch.full(want.shape, -1.0, device="cuda")
+    torch.cuda.synchronize()
+    for _ in range(2):
+        assert tomo.lib().tomo_forward_noalloc(C.byref(cfg), C.c_void_p(d_f.data_ptr()), C.c_void_p(d_rec.data_ptr()),
+                                               None) == tomo.OK
+    torch.cuda.synchronize()
+    assert np.array_equal(d_rec.cpu().numpy(), want)
+    assert np.abs(want).max() > 0

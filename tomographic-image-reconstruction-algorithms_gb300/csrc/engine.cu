@@ -104,7 +104,7 @@ struct tomo_ctx {
     int learned_backtrack = 0;   // retries of a rejected proposal at half the scale (tomo_run_learned)
     int learned_resume = 0;      // plain steps after which paused proposals resume (0: never)
     static constexpr int ZR = 4; // adjoint ring slots
-    static constexpr int UR = 4; // wavefield ring slots of the streamed sweeps
+    static constexpr int UR = STREAM_RING; // wavefield ring slots of the streamed sweeps
     TileMaps tmaps;              // TMA maps of hist, z, coef, dmap, rid (tile kernels)
     TileMaps tmaps_ck;           // the same with the slice maps over the checkpoint buffer (pass_layout)
     unsigned int* err_host = nullptr;   // tile kernels' wait time-out word (mapped pinned memory)
@@ -969,63 +969,24 @@ int64_t record_resident_pass(tomo_ctx* c, int mode, int g0, int ng) {
     return n;
 }
 
-// Steps of the next streamed launch when L remain: the last launch of a segment advances two or more
-// steps where the segment has them, so both slices of its end state come from one launch.
-int stream_steps(int L) { return L >= 6 || L == 4 ? 4 : L % 2 ? 1 : 2; }
-
-// The wavefield state of a streamed sweep: slices k-1 and k, each with its group stride.
-struct StreamState {
-    float *p0, *p1;
-    int64_t s0, s1;
-};
-
 // Forward steps of a streamed pass from slice k0 (state st) to slice k0 + T, L(q) of q >= qlo kept when
 // keep, the end state written to end0, end1 (null: the ring).  Returns the launches.
 int64_t stream_forward(tomo_ctx* c, StreamState& st, int k0, int T, int g0, int ng, bool keep, int qlo, float* gout, float* end0,
                        float* end1, int64_t endstride) {
-    int64_t n = 0;
-    const int64_t NS = c->NS, us = tomo_ctx::UR * NS;
-    while (T > 0) {
-        StreamFwd a{};
-        a.T = stream_steps(T);
-        a.coef = c->coefp;
-        a.dmap = c->dmapp;
-        a.in0 = st.p0;
-        a.in1 = st.p1;
-        a.in0stride = st.s0;
-        a.in1stride = st.s1;
-        if (T == a.T && end0) {
-            a.out0 = end0;
-            a.out1 = end1;
-            a.outstride = endstride;
-        } else {   // two ring slots the inputs are not in
-            float* free[2] = {nullptr, nullptr};
-            for (int k = 0, f = 0; k < tomo_ctx::UR && f < 2; ++k) {
-                float* s = c->ust + k * NS;
-                if (s != st.p0 && s != st.p1) free[f++] = s;
-            }
-            a.out0 = free[0];
-            a.out1 = free[1];
-            a.outstride = us;
-        }
-        a.hist = keep ? c->hist : nullptr;
-        a.hstride = (int64_t)c->S * NS;
-        a.ns = NS;
-        a.qlo = qlo;
-        a.k0 = k0;
-        a.g0 = g0;
-        a.ng = ng;
-        a.px = c->px;
-        a.gout = gout;
-        a.rec = StreamRec{c->rchan, c->rcell, c->rowstart};
-        launch_stream_fwd(c->dg, a, c->st);
-        ++n;
-        if (a.T == 1) st = StreamState{st.p1, a.out1, st.s1, a.outstride};
-        else st = StreamState{a.out0, a.out1, a.outstride, a.outstride};
-        k0 += a.T;
-        T -= a.T;
-    }
-    return n;
+    const int64_t NS = c->NS;
+    StreamFwd a{};
+    a.coef = c->coefp;
+    a.hist = keep ? c->hist : nullptr;
+    a.hstride = (int64_t)c->S * NS;
+    a.ns = NS;
+    a.qlo = qlo;
+    a.k0 = k0;
+    a.g0 = g0;
+    a.ng = ng;
+    a.px = c->px;
+    a.gout = gout;
+    a.rec = StreamRec{c->rchan, c->rcell, c->rowstart};
+    return launch_stream_steps(c->dg, a, st, T, c->ust, tomo_ctx::UR * NS, end0, end1, endstride, c->st);
 }
 
 // Adjoint steps of a streamed pass: z(kz0) .. z(kz0-T+1) from the state (p0 = z(kz0+2), p1 = z(kz0+1))

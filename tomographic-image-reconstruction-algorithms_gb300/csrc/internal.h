@@ -396,7 +396,7 @@ struct StreamRec {
     const int32_t *rchan, *rcell, *rowstart;   // receivers in row order (cells of the unpadded grid)
 };
 struct StreamFwd {
-    const float *coef, *dmap;       // framed
+    const float* coef;              // framed
     const float *in0, *in1;         // u(k0-1), u(k0)
     int64_t in0stride, in1stride;
     float *out0, *out1;             // u(k0+T-1) (T > 1), u(k0+T): not the inputs' slices
@@ -427,7 +427,17 @@ struct StreamAdj {
 };
 int stream_pitch(int nx);
 int64_t stream_slice(int nx, int ny);
+// The wavefield state of a streamed sweep: slices k-1 and k, each with its group stride.
+struct StreamState {
+    float *p0, *p1;
+    int64_t s0, s1;
+};
+constexpr int STREAM_RING = 4;      // wavefield slots a forward sweep goes round
 void launch_stream_fwd(const DevGeo& g, const StreamFwd& a, void* stream);
+// Forward steps from slice a.k0 (state st) to slice a.k0 + T through the ring (STREAM_RING slices of a.ns
+// floats per group, groups rstride apart); the end state goes to end0, end1 when given.  Returns the launches.
+int64_t launch_stream_steps(const DevGeo& g, StreamFwd a, StreamState& st, int T, float* ring, int64_t rstride, float* end0,
+                            float* end1, int64_t endstride, void* stream);
 void launch_stream_adj(const DevGeo& g, const StreamAdj& a, void* stream);
 void launch_resid_meas(const DevGeo& g, float* rr, const float* meas, int g0, int ng, double* part, void* stream);
 void launch_frame(float* dst, const float* src, int nx, int ny, void* stream);

@@ -10,13 +10,15 @@
 //
 // Grids that fit on chip (resident.cuh) are solved by one launch for all groups, which keeps the
 // wavefield in registers and uses the array for the coefficients and tables only: 128 x 128, 600
-// steps, 8 groups took 39.2 ms as a step and a gather launch per time step and group.  Larger grids
-// go a group at a time through the array's time slots.
+// steps, 8 groups took 39.2 ms as a step and a gather launch per time step and group and takes 0.24.
+// Larger grids go a group at a time through the array's time slots: benchmark-profile grids whose framed
+// slices fit the array by the streamed sweeps, four steps to a launch (launches are what bounds it; 300 x 330
+// 8.2 -> 3.8 us per step and group), the others by a step and a gather launch per time step.
 //
-// The scratch array g_scratch is a fixed kNoallocScratchBytes (about 5.1 MiB)
+// The scratch array g_scratch is a fixed kNoallocScratchBytes (about 5.6 MiB)
 // that every GPU loading this library holds until the process exits.  It holds
-// the two coefficient fields, the geometry tables and, for one emitter group at
-// a time, three forward time slots, so a call accepts grids of up to
+// the coefficient fields, the geometry tables and, for one emitter group at
+// a time, three forward time slots (four framed ones in a streamed solve), so a call accepts grids of up to
 // kNoallocMaxCells cells (512 x 512), kNoallocMaxChannels record channels and
 // kNoallocMaxSteps time steps, plus kNoallocMaxEmitters emitters (benchmark
 // profile) or kNoallocMaxGroups emission boxes (reference profile), and rejects
@@ -34,7 +36,7 @@
 // call's host-side tables after it returns.
 //
 // All calls share the one array and it keeps the last call's contents: each
-// call zeroes the two initial time slots it starts from and the output records,
+// call zeroes the time slots it starts from and the output records,
 // and rewrites everything else before reading it.  Calls that overlap on the
 // GPU (concurrent streams, or threads, on the same device) race on the array:
 // serialise them on one stream.
@@ -59,8 +61,11 @@ constexpr int kNoallocMaxEmitters = 4096;
 constexpr int kNoallocMaxSteps = 16384;
 constexpr int kNoallocMaxRows = 1024;      // grid rows of a cluster-resident solve
 
-// float region: 3 time slots + coefficient + edge coefficient + source table
-constexpr int64_t kFloats = 5 * kNoallocMaxCells + kNoallocMaxSteps;
+// float region: 3 time slots + coefficient + edge coefficient, or the framed slots and coefficient of a streamed
+// solve (528 x 536 + 128 floats each at 512 x 512); then the source table
+constexpr int64_t kFields = 5 * (int64_t)(528 * 536 + 128);
+constexpr int64_t kFloats = kFields + kNoallocMaxSteps;
+static_assert(kFields >= 5 * kNoallocMaxCells, "fields of the largest grid");
 // int region: receiver cells, emitter cells, emission boxes; for a cluster-resident solve receivers in row
 // order (channel, cell), the first of each row, and the reference profile's rows of each warp and row slots
 constexpr int64_t kInts = 3 * kNoallocMaxChannels + kNoallocMaxEmitters + 4 * kNoallocMaxGroups + 3 * (kNoallocMaxRows + 1);
@@ -138,7 +143,7 @@ extern "C" tomo_status tomo_forward_noalloc(const tomo_config* cfg, const float*
     float* slots = (float*)base;                       // 3 time slots
     float* coef = slots + 3 * kNoallocMaxCells;
     float* rcoef = coef + kNoallocMaxCells;
-    float* src = rcoef + kNoallocMaxCells;             // tables: source, then the integer tables behind it
+    float* src = slots + kFields;                      // tables: source, then the integer tables behind it
     cudaError_t e;
 #define NA_CU(x)                                     \
     do {                                             \
@@ -155,11 +160,13 @@ extern "C" tomo_status tomo_forward_noalloc(const tomo_config* cfg, const float*
     // a grid that fits on chip is solved by one launch for all groups
     std::vector<int32_t> chan, cell, rowstart, warps, slot;
     ResShape shape;
+    bool streamed = false;
     if (const char* off = std::getenv("TOMO_RESIDENT"); geo.ny <= kNoallocMaxRows && !(off && *off == '0')) {
         res_receivers(geo.rcv, geo.nx, geo.ny, chan, cell, rowstart);
         if (geo.ref) warps = ref_warps(geo.ny, geo.lo, geo.hi);
         shape = res_pick(geo.ref ? ref_shapes(geo.nx, geo.ny, warps, rowstart) : res_shapes(geo.nx, geo.ny, rowstart), geo.G);
         if (shape.cpl && res_held(shape) < 1) shape = ResShape{};
+        streamed = !shape.cpl && !geo.ref && (STREAM_RING + 1) * stream_slice(geo.nx, geo.ny) <= kFields;
     }
     // every table in one block of words behind the source table
     std::vector<uint32_t> words;
@@ -174,7 +181,7 @@ extern "C" tomo_status tomo_forward_noalloc(const tomo_config* cfg, const float*
     if (geo.ref) dg.box = put(geo.box.data(), 4 * (int64_t)geo.G);
     else dg.emit = put(geo.emit.data(), (int64_t)geo.G * geo.gs);
     ResFwd r{};
-    if (shape.cpl) {
+    if (shape.cpl || streamed) {
         r.rchan = put(chan.data(), (int64_t)chan.size());
         r.rcell = put(cell.data(), (int64_t)cell.size());
         r.rowstart = put(rowstart.data(), geo.ny + 1);
@@ -194,6 +201,29 @@ extern "C" tomo_status tomo_forward_noalloc(const tomo_config* cfg, const float*
     unsigned int* const err = (unsigned int*)put(&zero, 1);
     if ((s = put_words((uint32_t*)src, words.data(), (int64_t)words.size(), st)) != TOMO_OK) return s;
     NA_CU(cudaMemsetAsync(d_records, 0, sizeof(float) * (size_t)geo.G * nt * nch, st));
+    if (streamed) {
+        const int64_t ns = stream_slice(geo.nx, geo.ny);
+        float* const framed = slots + STREAM_RING * ns;
+        launch_coef(prof, d_f, slots, slots + N, N, cfg->courant, st);   // in the slots' place
+        launch_frame(framed, slots, geo.nx, geo.ny, st);
+        launch_zero_slots(slots, 1, STREAM_RING * ns, 0, 2 * ns, 2 * ns, st);   // all four, guard cells included
+        StreamFwd a{};
+        a.coef = framed;
+        a.ns = ns;
+        a.k0 = 1;
+        a.ng = 1;
+        a.px = stream_pitch(geo.nx);
+        a.rec = StreamRec{r.rchan, r.rcell, r.rowstart};
+        for (int g = 0; g < geo.G; ++g) {
+            if (g > 0) launch_zero_slots(slots, 1, STREAM_RING * ns, 0, ns, ns, st);   // u(0) = u(1) = 0
+            a.g0 = g;
+            a.gout = d_records + (int64_t)g * nt * nch;
+            StreamState u{slots, slots + ns, 0, 0};
+            launch_stream_steps(dg, a, u, geo.nt - 2, slots, 0, nullptr, nullptr, 0, st);
+        }
+        NA_CU(cudaGetLastError());
+        return TOMO_OK;
+    }
     launch_coef(prof, d_f, coef, rcoef, N, cfg->courant, st);
     if (shape.cpl) {
         r.coef = coef;
@@ -208,9 +238,7 @@ extern "C" tomo_status tomo_forward_noalloc(const tomo_config* cfg, const float*
         NA_CU(cudaGetLastError());
         return TOMO_OK;
     }
-    // otherwise a group at a time: a strip launch per step, which also gathers the slice before (widths of
-    // whole 128-bit vectors), or a step and a gather launch
-    const bool strip = !geo.ref && geo.nx % 4 == 0;   // k_fwd_strip reads none of the receiver maps
+    // otherwise a group at a time, a step and a gather launch per step
     auto at = [&](int k) { return slots + (int64_t)(k % 3) * N; };
     for (int g = 0; g < geo.G; ++g) {
         launch_zero_slots(slots, 1, 3 * N, 0, N, N, st);   // u(0) = u(1) = 0
@@ -224,14 +252,7 @@ extern "C" tomo_status tomo_forward_noalloc(const tomo_config* cfg, const float*
             fs.k = k;
             fs.g0 = g;
             fs.ng = 1;
-            if (strip) {
-                fs.gk = k;
-                fs.gout = out;
-                launch_fwd_strip(8, dg, coef, fs, st);
-                if (k < geo.nt - 2) continue;
-            } else {
-                launch_fwd_step(prof, dg, coef, rcoef, fs, st);
-            }
+            launch_fwd_step(prof, dg, coef, rcoef, fs, st);
             GatherStep gs{};
             gs.u = at(k + 1);
             gs.gstride = 3 * N;

@@ -563,6 +563,38 @@ void launch_stream_fwd(const DevGeo& g, const StreamFwd& a, void* st) {
     else if (a.T == 2) src ? go_fwd<2, true>(g, a, st) : go_fwd<2, false>(g, a, st);
     else src ? go_fwd<1, true>(g, a, st) : go_fwd<1, false>(g, a, st);
 }
+int64_t launch_stream_steps(const DevGeo& g, StreamFwd a, StreamState& st, int T, float* ring, int64_t rstride, float* end0,
+                            float* end1, int64_t endstride, void* stream) {
+    int64_t n = 0;
+    for (; T > 0; T -= a.T, ++n) {
+        // the last launch advances two or more steps where there are any, so both slices of the end state come
+        // from one launch
+        a.T = T >= 6 || T == 4 ? 4 : T % 2 ? 1 : 2;
+        a.in0 = st.p0;
+        a.in1 = st.p1;
+        a.in0stride = st.s0;
+        a.in1stride = st.s1;
+        if (T == a.T && end0) {
+            a.out0 = end0;
+            a.out1 = end1;
+            a.outstride = endstride;
+        } else {   // two ring slots the inputs are not in
+            float* free[2] = {nullptr, nullptr};
+            for (int k = 0, f = 0; k < STREAM_RING && f < 2; ++k) {
+                float* s = ring + k * a.ns;
+                if (s != st.p0 && s != st.p1) free[f++] = s;
+            }
+            a.out0 = free[0];
+            a.out1 = free[1];
+            a.outstride = rstride;
+        }
+        launch_stream_fwd(g, a, stream);
+        if (a.T == 1) st = StreamState{st.p1, a.out1, st.s1, a.outstride};
+        else st = StreamState{a.out0, a.out1, a.outstride, a.outstride};
+        a.k0 += a.T;
+    }
+    return n;
+}
 void launch_stream_adj(const DevGeo& g, const StreamAdj& a, void* st) {
     if (a.T == 4) go_adj<4>(g, a, st);
     else if (a.T == 2) go_adj<2>(g, a, st);

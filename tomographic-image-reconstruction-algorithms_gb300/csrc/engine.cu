@@ -90,7 +90,7 @@ struct tomo_ctx {
     std::vector<int32_t> h_rowstart, h_warps;
     int32_t *warps = nullptr, *rowslot = nullptr;   // reference profile: rows of each warp, slot of each row
     std::vector<ResShape> res_cands;   // every shape that holds a group (tune_resident times them)
-    bool res_tuned = false;
+    bool res_tuned[2] = {false, false}, stream_tuned[2] = {false, false};   // for passes of one group, of more
     // several steps per launch on grids that do not fit on chip (stream.cu): possible, and chosen for passes
     // of P groups and of one; framed slices of pitch px
     bool stream_ok = false, stream = false, stream1 = false;
@@ -1364,17 +1364,42 @@ struct LayoutScope {
     }
 };
 
-// Picks the cluster shapes of the resident sweeps, for passes of P groups and of one, by timing a
-// forward and an adjoint segment of every shape that holds a group on this problem: which of them is
-// fastest depends on how many clusters the GPU holds at once, which only the GPU knows.  All shapes
-// give the same bits.  TOMO_RES_SHAPE="cs,rpw" fixes the choice; TOMO_TUNE_CACHE reuses or records
+// A recorded choice: the `n` numbers after `key` on a line of the cache file that `fits` accepts.
+template <typename Fits>
+bool read_choice(const char* cache, const char* key, int n, int* v, Fits fits) {
+    FILE* fp = cache && *cache ? std::fopen(cache, "r") : nullptr;
+    if (!fp) return false;
+    char line[512];
+    bool hit = false;
+    const size_t len = std::strlen(key);
+    while (!hit && std::fgets(line, sizeof line, fp))
+        if (std::strncmp(line, key, len) == 0 && line[len] == ' ')
+            hit = std::sscanf(line + len, "%d %d", &v[0], &v[1]) >= n && fits();
+    std::fclose(fp);
+    return hit;
+}
+void write_choice(const char* cache, const char* key, const char* value) {
+    FILE* fp = cache && *cache ? std::fopen(cache, "a") : nullptr;
+    if (!fp) return;
+    std::fprintf(fp, "%s %s\n", key, value);
+    std::fclose(fp);
+}
+
+// Picks the cluster shape of the resident sweeps for passes of one group or of more (up to P), by timing a
+// forward and an adjoint segment of shapes that hold a group on this problem: which of them is fastest
+// depends on how many clusters the GPU holds at once, which only the GPU knows.  Of the shapes with as many rows
+// per warp, a cluster of fewer blocks takes longer over a step, so it is worth a trial only if it saves a round
+// of clusters; of those that hold all groups at once the two largest are tried.  2 to 6 trials of up to 26
+// shapes: all of them took 15 to 55 ms of a context's first pass, and found the same shapes to 1 %.
+// All shapes give the same bits.  TOMO_RES_SHAPE="cs,rpw" fixes the choice; TOMO_TUNE_CACHE reuses or records
 // it; TOMO_TUNE_LOG prints each candidate's time.
-tomo_status tune_resident(tomo_ctx* c) {
-    if (c->res_tuned || !c->res.cpl) return TOMO_OK;
-    c->res_tuned = true;
-    const auto& cands = c->res_cands;
+tomo_status tune_resident(tomo_ctx* c, int groups) {
+    const int which = groups > 1 ? 1 : 0, ng = which ? c->P : 1;
+    if (!c->res.cpl || c->res_tuned[which]) return TOMO_OK;
+    c->res_tuned[which] = true;
+    ResShape& pick = which ? c->res : c->res1;
     auto find = [&](int cs, int rpw) -> const ResShape* {
-        for (const ResShape& s : cands)
+        for (const ResShape& s : c->res_cands)
             if (s.cs == cs && s.rpw == rpw) return &s;
         return nullptr;
     };
@@ -1382,75 +1407,67 @@ tomo_status tune_resident(tomo_ctx* c) {
         int cs = 0, rpw = 0;
         if (std::sscanf(e, "%d,%d", &cs, &rpw) == 2)
             if (const ResShape* s = find(cs, rpw)) {
-                c->res = c->res1 = *s;
+                pick = *s;
                 return TOMO_OK;
             }
     }
     const Geometry& g = c->geo;
     const char* cache = std::getenv("TOMO_TUNE_CACHE");
     char key[160];
-    std::snprintf(key, sizeof key, "tomo-res-1 %d %d %d %d %d %d", g.cfg.profile, g.nx, g.ny, g.nt, c->P, c->S);
-    if (cache && *cache)
-        if (FILE* fp = std::fopen(cache, "r")) {
-            char line[512];
-            bool hit = false;
-            while (!hit && std::fgets(line, sizeof line, fp)) {
-                int v[4];
-                const size_t n = std::strlen(key);
-                if (std::strncmp(line, key, n) != 0 || line[n] != ' ' ||
-                    std::sscanf(line + n, "%d %d %d %d", &v[0], &v[1], &v[2], &v[3]) != 4)
-                    continue;
-                const ResShape *p = find(v[0], v[1]), *o = find(v[2], v[3]);
-                if (p && o) {
-                    c->res = *p;
-                    c->res1 = *o;
-                    hit = true;
-                }
-            }
-            std::fclose(fp);
-            if (hit) return TOMO_OK;
-        }
-    const bool tlog = std::getenv("TOMO_TUNE_LOG") != nullptr;
-    for (int which = 0; which < (c->P > 1 ? 2 : 1); ++which) {
-        const int ng = which == 0 ? 1 : c->P;
-        // long enough that a launch's set-up does not decide, where a step is short
-        const int T = std::min(std::min(c->K, g.nt - 2), (double)ng * g.N < 1e6 ? 160 : 48);
-        float best = 1e30f;
-        for (const ResShape& s : cands) {
-            if (res_held(s) < 1) continue;
-            float ms = 1e30f;
-            for (int pass = 0; pass < 3; ++pass) {   // the first warms up
-                ResFwd f = res_fwd_args(c, s, 1, T, 0, ng);
-                f.hist = c->hist;
-                f.qlo = 1;
-                ResAdj a = res_adj_args(c, s, g.ref ? T : T + 1, T, 0, ng);
-                a.qlo = 1;
-                a.first = true;
-                CU(c, cudaEventRecord(c->ev0, c->st));
-                launch_res_fwd(s, c->dg, f, c->st);
-                launch_res_adj(s, c->dg, a, c->st);
-                CU(c, cudaEventRecord(c->ev1, c->st));
-                CU(c, cudaEventSynchronize(c->ev1));
-                CU(c, cudaGetLastError());
-                float t = 0.f;
-                CU(c, cudaEventElapsedTime(&t, c->ev0, c->ev1));
-                if (pass > 0) ms = std::min(ms, t);
-            }
-            if (tlog)
-                std::fprintf(stderr, "tomo tune: resident, %d groups: clusters of %d, %d warps of %d rows: %.2f us per %d steps\n",
-                             ng, s.cs, s.warps, s.rpw, 1e3 * ms, T);
-            if (ms < best) {
-                best = ms;
-                (which == 0 ? c->res1 : c->res) = s;
-            }
-        }
-        if (which == 0) c->res = c->res1;
+    std::snprintf(key, sizeof key, "tomo-res-1 %d %d %d %d %d %d", g.cfg.profile, g.nx, g.ny, g.nt, ng, c->S);
+    int v[2];
+    if (read_choice(cache, key, 2, v, [&] { return find(v[0], v[1]) != nullptr; })) {
+        pick = *find(v[0], v[1]);
+        return TOMO_OK;
     }
-    if (cache && *cache)
-        if (FILE* fp = std::fopen(cache, "a")) {
-            std::fprintf(fp, "%s %d %d %d %d\n", key, c->res.cs, c->res.rpw, c->res1.cs, c->res1.rpw);
-            std::fclose(fp);
+    std::vector<ResShape> cands;
+    int rpw = 0, least = 0, same = 0;   // of the rows per warp at hand: fewest rounds so far, shapes that take as many
+    for (const ResShape& s : c->res_cands) {   // by rows per warp, larger clusters first
+        const int held = res_held(s);
+        if (held < 1) continue;
+        const int rounds = (ng + held - 1) / held;
+        if (s.rpw != rpw) least = 1 << 30;
+        rpw = s.rpw;
+        if (rounds > least || (rounds == least && (rounds > 1 || same == 2))) continue;
+        same = rounds < least ? 1 : 2;
+        least = rounds;
+        cands.push_back(s);
+    }
+    const bool tlog = std::getenv("TOMO_TUNE_LOG") != nullptr;
+    // long enough that a launch's set-up does not decide, where a step is short
+    const int T = std::min(std::min(c->K, g.nt - 2), (double)ng * g.N < 1e6 ? 96 : (double)ng * g.N < 2e6 ? 32 : 16);
+    float best = 1e30f;
+    for (const ResShape& s : cands) {
+        float ms = 1e30f;
+        for (int pass = 0; pass < 3; ++pass) {   // the first warms up
+            ResFwd f = res_fwd_args(c, s, 1, T, 0, ng);
+            f.hist = c->hist;
+            f.qlo = 1;
+            ResAdj a = res_adj_args(c, s, g.ref ? T : T + 1, T, 0, ng);
+            a.qlo = 1;
+            a.first = true;
+            CU(c, cudaEventRecord(c->ev0, c->st));
+            launch_res_fwd(s, c->dg, f, c->st);
+            launch_res_adj(s, c->dg, a, c->st);
+            CU(c, cudaEventRecord(c->ev1, c->st));
+            CU(c, cudaEventSynchronize(c->ev1));
+            CU(c, cudaGetLastError());
+            float t = 0.f;
+            CU(c, cudaEventElapsedTime(&t, c->ev0, c->ev1));
+            if (pass > 0) ms = std::min(ms, t);
+            if (pass == 1 && t > 0.2f) break;    // long enough to be steady
         }
+        if (tlog)
+            std::fprintf(stderr, "tomo tune: resident, %d groups: clusters of %d, %d warps of %d rows: %.2f us per %d steps\n",
+                         ng, s.cs, s.warps, s.rpw, 1e3 * ms, T);
+        if (ms < best) {
+            best = ms;
+            pick = s;
+        }
+    }
+    char value[32];
+    std::snprintf(value, sizeof value, "%d %d", pick.cs, pick.rpw);
+    write_choice(cache, key, value);
     return TOMO_OK;
 }
 
@@ -1478,14 +1495,15 @@ void enqueue_steps(tomo_ctx* c, int which, int k0, int steps, int ng, bool keep)
             const int T = std::min(steps - t, c->K);
             StreamState u{c->ust, c->ust + c->NS, tomo_ctx::UR * c->NS, tomo_ctx::UR * c->NS};
             StreamState z{c->z, c->z + c->NS, tomo_ctx::ZR * c->NS, tomo_ctx::ZR * c->NS};
-            if (which == 0) stream_forward(c, u, k0, T, 0, ng, keep, k0, nullptr, nullptr, nullptr, 0);
+            // a sweep writes its records in the steps that keep no history (all but the last chunk's)
+            if (which == 0) stream_forward(c, u, k0, T, 0, ng, keep, k0, keep ? nullptr : c->rr, nullptr, nullptr, 0);
             else stream_adjoint(c, z, k0 + T, T, 0, ng, k0);
             t += T;
-        } else if (which == 0 && c->tile_fwd) {
+        } else if (which == 0 && (ng == 1 ? c->tile_fwd1 : c->tile_fwd)) {
             const int T = tile_fwd_steps(c, steps - t);
             launch_fwd_tile(c->dg, c->tmaps, tile_fwd_args(c, k0 + t, T, 0, ng), c->st);
             t += T;
-        } else if (which == 1 && c->tile_adj) {
+        } else if (which == 1 && (ng == 1 ? c->tile_adj1 : c->tile_adj)) {
             const int T = tile_adj_steps(steps - t);
             launch_adj_tile(c->dg, c->tmaps, tile_adj_args(c, k0 + steps - t, T, 0, ng), c->st);
             t += T;
@@ -1507,56 +1525,78 @@ void enqueue_steps(tomo_ctx* c, int which, int k0, int steps, int ng, bool keep)
     }
 }
 
-// Chooses between the streamed sweeps and the per-step (or tile) kernels autotune has picked, for
-// passes of P groups and of one, by timing steps of each: per step a pass costs a forward step
-// (streamed: with the history kept, in the last chunk only), for all chunks but one a recomputed forward
-// step with the history, and an adjoint step.  Sweeps too short for a trial keep the strip kernels where
-// the width allows them (a multiple of 4) and are streamed otherwise.  TOMO_STREAM=1 fixes the choice.
-tomo_status tune_stream(tomo_ctx* c) {
-    if (c->tuned) return TOMO_OK;
+// Chooses between the streamed sweeps and the per-step (or tile) kernels autotune picks, for passes of one
+// group or of more (up to P).  Streamed without a trial: passes whose slices of all groups are a quarter of the
+// L2 or more, which are bound by bytes (iterations at 512 x 512, 32 groups: 134 -> 120 ms, 2048 x 2048, 8: 77 ->
+// 56; the trials and autotune's took 170 ms of a context's first pass), and widths that are not a multiple of 4,
+// which only the per-cell kernels take otherwise (403 x 390, 8 groups: 7.0 -> 3.8 ms together, 21.4 -> 17.4 one by
+// one).  Else steps of each are timed: a step of a pass costs a forward step with records, for all chunks but
+// one a recomputed forward step with the history, and an adjoint step; small passes are faster in tiles, from
+// the L2 (one group of 512 x 512: 0.95 + 1.28 us per step against 2.97 + 2.63; 8 groups: 3.6 + 7.2 against 4.0 +
+// 6.1).  Sweeps too short for a trial keep the strip kernels.  TOMO_STREAM=1 fixes the choice; TOMO_TUNE_CACHE
+// reuses or records it.
+tomo_status tune_stream(tomo_ctx* c, int groups) {
+    const int one = groups > 1 ? 0 : 1, ng = one ? 1 : c->P;
+    bool& pick = one ? c->stream1 : c->stream;
+    if (!c->stream_ok) return autotune(c);
+    if (c->stream_tuned[one ? 0 : 1]) return TOMO_OK;
+    c->stream_tuned[one ? 0 : 1] = true;
     const char* e = std::getenv("TOMO_STREAM");
-    const int steps = 16, nt = c->geo.nt;
-    if (c->stream_ok && ((!c->strip && nt < 4 * steps) || (e && *e == '1'))) {
-        c->tuned = c->stream = c->stream1 = true;
+    const int nt = c->geo.nt, steps = std::min(64, nt / 4);
+    pick = true;
+    if ((e && *e == '1') || !c->strip || 4.0 * ng * c->geo.N >= (32 << 20)) return TOMO_OK;
+    pick = false;
+    TRY(autotune(c));
+    if (nt < 64) return TOMO_OK;
+    const char* cache = std::getenv("TOMO_TUNE_CACHE");
+    char key[160];
+    std::snprintf(key, sizeof key, "tomo-stream-1 %d %d %d %d %d", c->geo.nx, c->geo.ny, nt, ng, c->K);
+    int v[2];
+    if (read_choice(cache, key, 1, v, [] { return true; })) {
+        pick = v[0] != 0;
         return TOMO_OK;
     }
-    TRY(autotune(c));
-    if (!c->stream_ok || nt < 4 * steps) return TOMO_OK;
     const int k0 = nt / 2 - steps;
     const double again = (double)(c->nchunk - 1) / c->nchunk;
-    auto time_steps = [&](int which, int ng, bool keep, double& ms) -> tomo_status {
+    // replayed from a graph, as passes are: issued one by one, short launches wait for the host (one group of
+    // 512 x 512: 8.4 us per step of the tile kernels, 2.7 in a pass)
+    auto time_steps = [&](int which, bool keep, double& ms) -> tomo_status {
+        cudaGraph_t graph = nullptr;
+        cudaGraphExec_t exec = nullptr;
+        CU(c, cudaStreamBeginCapture(c->st, cudaStreamCaptureModeThreadLocal));
+        enqueue_steps(c, which, k0, steps, ng, keep);
+        const cudaError_t ec = cudaStreamEndCapture(c->st, &graph);
+        const cudaError_t ei = ec == cudaSuccess ? cudaGraphInstantiate(&exec, graph, 0) : ec;
+        if (graph) cudaGraphDestroy(graph);
+        CU(c, ei);
         ms = 1e30;
-        for (int pass = 0; pass < 3; ++pass) {   // the first warms up
-            CU(c, cudaEventRecord(c->ev0, c->st));
-            enqueue_steps(c, which, k0, steps, ng, keep);
-            CU(c, cudaEventRecord(c->ev1, c->st));
-            CU(c, cudaEventSynchronize(c->ev1));
-            CU(c, cudaGetLastError());
+        cudaError_t er = cudaSuccess;
+        for (int pass = 0; pass < 3 && er == cudaSuccess; ++pass) {   // the first warms up
             float t = 0.f;
-            CU(c, cudaEventElapsedTime(&t, c->ev0, c->ev1));
+            cudaEventRecord(c->ev0, c->st);
+            cudaGraphLaunch(exec, c->st);
+            cudaEventRecord(c->ev1, c->st);
+            er = cudaEventSynchronize(c->ev1);
+            if (er == cudaSuccess) er = cudaEventElapsedTime(&t, c->ev0, c->ev1);
             if (pass > 0) ms = std::min(ms, (double)t);
         }
+        cudaGraphExecDestroy(exec);
+        CU(c, er);
         return TOMO_OK;
     };
-    bool better[2] = {false, false};
-    for (int one = 0; one < 2; ++one) {
-        const int ng = one ? 1 : c->P;
-        double f = 0.0, a = 0.0, fn = 0.0, fk = 0.0, b = 0.0;
-        c->stream = c->stream1 = false;
-        TRY(time_steps(0, ng, true, f));
-        TRY(time_steps(1, ng, true, a));
-        c->stream = c->stream1 = true;
-        TRY(time_steps(0, ng, false, fn));
-        TRY(time_steps(0, ng, true, fk));
-        TRY(time_steps(1, ng, true, b));
-        better[one] = again * fn + fk + b < f * (1.0 + again) + a;
-        if (std::getenv("TOMO_TUNE_LOG"))
-            std::fprintf(stderr, "tomo tune: %d groups, us per step: per-step kernels forward %.2f adjoint %.2f, streamed forward "
-                         "%.2f (with history %.2f) adjoint %.2f\n", ng, 1e3 * f / steps, 1e3 * a / steps, 1e3 * fn / steps,
-                         1e3 * fk / steps, 1e3 * b / steps);
-    }
-    c->stream = better[0];
-    c->stream1 = c->P > 1 ? better[1] : better[0];
+    double f = 0.0, a = 0.0, fn = 0.0, fk = 0.0, b = 0.0;
+    TRY(time_steps(0, true, f));
+    TRY(time_steps(1, true, a));
+    pick = true;
+    TRY(time_steps(0, false, fn));
+    TRY(time_steps(0, true, fk));
+    TRY(time_steps(1, true, b));
+    pick = again * fn + fk + b < 0.92 * (f * (1.0 + again) + a);   // the steps with sources gain less
+    if (std::getenv("TOMO_TUNE_LOG"))
+        std::fprintf(stderr, "tomo tune: %d groups, us per step: per-step kernels forward %.2f adjoint %.2f, streamed forward "
+                     "%.2f (with history %.2f) adjoint %.2f\n", ng, 1e3 * f / steps, 1e3 * a / steps, 1e3 * fn / steps,
+                     1e3 * fk / steps, 1e3 * b / steps);
+    write_choice(cache, key, pick ? "1" : "0");
     return TOMO_OK;
 }
 
@@ -1564,8 +1604,7 @@ tomo_status run_pass(tomo_ctx* c, int mode, int g0, int ng) {
     const auto key = std::make_tuple(mode, g0, ng);
     auto it = c->graphs.find(key);
     if (it == c->graphs.end()) {
-        if (c->res.cpl) TRY(mode == MODE_ILLUM ? autotune(c) : tune_resident(c));
-        else TRY(tune_stream(c));
+        TRY(mode == MODE_ILLUM ? autotune(c) : c->res.cpl ? tune_resident(c, ng) : tune_stream(c, ng));
         LayoutScope layout(c, pass_layout(c, mode, ng));
         cudaGraph_t graph = nullptr;
         CU(c, cudaStreamBeginCapture(c->st, cudaStreamCaptureModeThreadLocal));
@@ -1644,7 +1683,8 @@ tomo_status apply_plan(tomo_ctx* c, const Plan& p) {
     c->release(&c->ust);
     c->release(&c->corrp);
     set_plan(c, p);
-    c->tuned = c->res_tuned = false;
+    c->tuned = false;
+    for (int k = 0; k < 2; ++k) c->res_tuned[k] = c->stream_tuned[k] = false;
     ++c->gen;
     TRY(alloc_plan_buffers(c));
     encode_maps(c);
@@ -1975,9 +2015,11 @@ tomo_status iterate_batch_graph(tomo_ctx** ctxs, int n, int method, const tomo_s
     // kernel choices first: the autotuner times trial passes, which a recording cannot hold
     for (int i = 0; i < n; ++i) {
         tomo_ctx* c = ctxs[i];
-        if (c->res.cpl ? !c->res_tuned : !c->tuned) {
+        for (const int ng : {c->P, c->geo.G % c->P}) {   // whole passes and the last one
+            const bool done = c->res.cpl ? c->res_tuned[ng > 1] : c->stream_ok ? c->stream_tuned[ng > 1] : c->tuned;
+            if (ng == 0 || done) continue;
             launch_coef(c->geo.cfg.profile, c->f, c->coef, c->rcoef, c->geo.N, c->geo.cfg.courant, c->st);
-            TRY(c->res.cpl ? tune_resident(c) : tune_stream(c));
+            TRY(c->res.cpl ? tune_resident(c, ng) : tune_stream(c, ng));
         }
     }
     uint64_t sbits = 0;
@@ -2649,7 +2691,7 @@ tomo_status tomo_time_kernel(tomo_ctx* c, int32_t which, int32_t steps, double* 
     steps = std::min(steps, nt - 4);
     const int k0 = std::max(2, (nt - steps) / 2);
     launch_coef(prof, c->f, c->coef, c->rcoef, N, g.cfg.courant, c->st);
-    TRY(c->res.cpl ? tune_resident(c) : tune_stream(c));
+    TRY(c->res.cpl ? tune_resident(c, ng) : tune_stream(c, ng));
     // the steps are captured into a graph and replayed, as the iterations run them, so the time
     // per step carries the launch gaps of graph replay, not of stream launches
     cudaGraph_t graph = nullptr;

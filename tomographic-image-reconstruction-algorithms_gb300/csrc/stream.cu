@@ -53,7 +53,7 @@ constexpr int AW = 64, AOWN = AW - 2 * AH;      // adjoint strip
 constexpr int MAXR = 128;        // rows of a band at most
 constexpr int FD = 6, FC = 12;   // forward ring slots: slices, coefficient (groups of 3)
 constexpr int AD = 3, AC = 9;    // adjoint ring slots
-constexpr int NREC = 64;         // receivers of a warp's strip kept in shared memory
+constexpr int NREC = 128;        // receivers of a warp's strip kept in shared memory
 
 __device__ __forceinline__ uint32_t saddr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void cp16(uint32_t dst, const float* src) {

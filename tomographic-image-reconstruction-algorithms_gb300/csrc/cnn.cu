@@ -376,7 +376,7 @@ __global__ void __launch_bounds__(192, 1) k_wgrad_tc(const __grid_constant__ CUt
                 for (int m = 0; m < copies; ++m) {
                     unsigned char* dst = xs + (m == 0 ? s : R + s) * NPL * PLANE;
                     for (int dx = 0; dx < 3; ++dx)   // one box: every chunk of the row, shifted by dx
-                        tma_load_5d(dst + dx * NCHX * PLANE, &x_map, 0, x0 + dx - 1, 0, yy, b, &xfull[s]);
+                        tma_load_4d(dst + dx * NCHX * PLANE, &x_map, 2 * (x0 + dx - 1), 0, yy, b, &xfull[s]);
                 }
                 ++q;
                 return true;
@@ -385,7 +385,7 @@ __global__ void __launch_bounds__(192, 1) k_wgrad_tc(const __grid_constant__ CUt
                 const int s = qd % RD;
                 if (qd >= RD && !role_wait(&dempty[s], (uint32_t)(qd / RD - 1) & 1u, a.wait_ns, abort)) return false;
                 mbar_expect_tx(&dfull[s], (uint32_t)S::DSLOT);
-                tma_load_5d(ds + s * S::DSLOT, &d_map, 0, x0, 0, yy, b, &dfull[s]);
+                tma_load_4d(ds + s * S::DSLOT, &d_map, 2 * x0, 0, yy, b, &dfull[s]);
                 ++qd;
                 return true;
             };
@@ -497,12 +497,41 @@ __global__ void k_pack_input(const float* __restrict__ feat, __nv_bfloat16* __re
     }
 }
 
+// Sum over a block of 256 threads, the same tree in every block.
+__device__ __forceinline__ double block_sum(double v, double* red) {
+    red[threadIdx.x] = v;
+    __syncthreads();
+    for (int s = 128; s > 0; s >>= 1) {
+        if (threadIdx.x < s) red[threadIdx.x] += red[threadIdx.x + s];
+        __syncthreads();
+    }
+    v = red[0];
+    __syncthreads();
+    return v;
+}
+__device__ __forceinline__ double block_total(const double* part, int n, double* red) {
+    double v = 0.0;
+    for (int i = threadIdx.x; i < n; i += 256) v += part[i];
+    return block_sum(v, red);
+}
+// Partial sums of the mask, in FP64.  (Copied to the host and added up there, 1 M pixels took 0.83 ms of a
+// gradient's 1.75.)
+__global__ void __launch_bounds__(256) k_mask_sum(const float* __restrict__ msk, int64_t n, double* __restrict__ part) {
+    __shared__ double red[256];
+    double acc = 0.0;
+    for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < n; p += (int64_t)gridDim.x * blockDim.x) acc += msk[p];
+    acc = block_sum(acc, red);
+    if (threadIdx.x == 0) part[blockIdx.x] = acc;
+}
+
 // Masked MSE: loss partial per block; dout = 2 mask (out - tgt) / msum, also packed as BF16
 // channels (dh, dl, dh, 0 ...) with dh + dl = dout to 16 bits, the output layer's gradient input.
 __global__ void __launch_bounds__(256) k_loss(const float* __restrict__ out, const float* __restrict__ tgt,
-                                             const float* __restrict__ msk, int64_t n, int W, float inv_msum,
+                                             const float* __restrict__ msk, int64_t n, int W,
                                              float* __restrict__ dout, __nv_bfloat16* __restrict__ dpk,
                                              double* __restrict__ part) {
+    __shared__ double red[256];
+    const float inv_msum = (float)(1.0 / block_total(part + gridDim.x, gridDim.x, red));   // k_mask_sum's partials
     double acc = 0.0;
     for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < n; p += (int64_t)gridDim.x * blockDim.x) {
         const float e = (out[p] - tgt[p]) * msk[p];
@@ -518,34 +547,34 @@ __global__ void __launch_bounds__(256) k_loss(const float* __restrict__ out, con
         *reinterpret_cast<uint4*>(o) = q0;
         *reinterpret_cast<uint4*>(o + (int64_t)W * 8) = make_uint4(0u, 0u, 0u, 0u);
     }
-    __shared__ double red[256];
-    red[threadIdx.x] = acc;
-    __syncthreads();
-    for (int s = 128; s > 0; s >>= 1) {
-        if (threadIdx.x < s) red[threadIdx.x] += red[threadIdx.x + s];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) part[blockIdx.x] = red[0];
+    acc = block_sum(acc, red);
+    if (threadIdx.x == 0) part[blockIdx.x] = acc;
 }
 
 // dst[j] = sum over blocks of part[blk][j], fixed order.
-__global__ void k_reduce_parts(const float* __restrict__ part, int nblk, int nout, float* __restrict__ dst) {
-    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < nout; j += gridDim.x * blockDim.x) {
-        float acc = 0.f;
-        for (int b = 0; b < nblk; ++b) acc += part[(int64_t)b * nout + j];
-        dst[j] = acc;
+// Sum of the blocks' partials: 8 threads to an output, each every eighth block, combined in fixed order (one
+// thread to an output waited on its 152 loads: 14.6 us for a layer).
+__global__ void __launch_bounds__(256) k_reduce_parts(const float* __restrict__ part, int nblk, int nout, float* __restrict__ dst) {
+    __shared__ float red[8][32];
+    const int o = threadIdx.x & 31, k = threadIdx.x >> 5, j = blockIdx.x * 32 + o;
+    float acc = 0.f;
+    if (j < nout) {
+#pragma unroll 4
+        for (int b = k; b < nblk; b += 8) acc += part[(int64_t)b * nout + j];
+    }
+    red[k][o] = acc;
+    __syncthreads();
+    if (k == 0 && j < nout)
+        dst[j] = ((red[0][o] + red[1][o]) + (red[2][o] + red[3][o])) + ((red[4][o] + red[5][o]) + (red[6][o] + red[7][o]));
+}
+// total[0], total[1]: sums of the loss and mask partials.
+__global__ void __launch_bounds__(256) k_totals(const double* __restrict__ part, int n, double* __restrict__ total) {
+    __shared__ double red[256];
+    for (int k = 0; k < 2; ++k) {
+        const double v = block_total(part + k * n, n, red);
+        if (threadIdx.x == 0) total[k] = v;
     }
 }
-
-__global__ void k_sum_double(const double* __restrict__ part, int n, double* __restrict__ out) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        double acc = 0.0;
-        for (int i = 0; i < n; ++i) acc += part[i];
-        *out = acc;
-    }
-}
-
-// Adam (bias-corrected) on the FP32 master parameters.
 __global__ void k_adam(float* __restrict__ w, float* __restrict__ m, float* __restrict__ v, const float* __restrict__ grad,
                        int n, float lr, float b1, float b2, float eps, float c1, float c2) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -656,15 +685,26 @@ bool encode_act_map(unsigned char out[128], const __nv_bfloat16* base, int C, in
     const EncodeTiled fn = reinterpret_cast<EncodeTiled>(tensor_map_encoder());
     if (!fn || C % 8 != 0) return false;
     CUtensorMap m;
-    // blocked layout [b][y][C / 8][x][8]: dimensions (channel in chunk, x, chunk, y, image)
     const cuuint64_t nch = (cuuint64_t)C / 8;
-    const cuuint64_t dims[5] = {8u, (cuuint64_t)W, nch, (cuuint64_t)H, (cuuint64_t)B};
-    const cuuint64_t strides[4] = {16u, (cuuint64_t)W * 16u, nch * W * 16u, (cuuint64_t)H * nch * W * 16u};
-    const cuuint32_t box[5] = {8u, (cuuint32_t)(conv_box ? PX : TX), (cuuint32_t)nch, 1u, 1u};
-    const cuuint32_t estr[5] = {1u, 1u, 1u, 1u, 1u};
-    const CUresult r = fn(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5u, const_cast<__nv_bfloat16*>(base), dims, strides,
-                          box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                          CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    CUresult r;
+    if (conv_box) {
+        // blocked layout [b][y][C / 8][x][8]: dimensions (channel in chunk, x, chunk, y, image)
+        const cuuint64_t dims[5] = {8u, (cuuint64_t)W, nch, (cuuint64_t)H, (cuuint64_t)B};
+        const cuuint64_t strides[4] = {16u, (cuuint64_t)W * 16u, nch * W * 16u, (cuuint64_t)H * nch * W * 16u};
+        const cuuint32_t box[5] = {8u, (cuuint32_t)PX, (cuuint32_t)nch, 1u, 1u};
+        const cuuint32_t estr[5] = {1u, 1u, 1u, 1u, 1u};
+        r = fn(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5u, const_cast<__nv_bfloat16*>(base), dims, strides, box, estr,
+               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    } else {
+        const cuuint64_t dims[4] = {2 * (cuuint64_t)W, nch, (cuuint64_t)H, (cuuint64_t)B};
+        const cuuint64_t strides[3] = {(cuuint64_t)W * 16u, nch * W * 16u, (cuuint64_t)H * nch * W * 16u};
+        const cuuint32_t box[4] = {2u * TX, (cuuint32_t)nch, 1u, 1u};
+        const cuuint32_t estr[4] = {1u, 1u, 1u, 1u};
+        r = fn(&m, CU_TENSOR_MAP_DATA_TYPE_UINT64, 4u, const_cast<__nv_bfloat16*>(base), dims, strides, box, estr,
+               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    }
     if (r != CUDA_SUCCESS) return false;
     std::memcpy(out, &m, sizeof m);
     return true;
@@ -705,13 +745,14 @@ void wgrad(WgradKind kind, const void* x_map, const void* d_map, float* part, in
         nout = WgradShape<32, 16>::NOUT;
         break;
     }
-    k_reduce_parts<<<blocks_for(nout, 256), 256, 0, st>>>(part, nblk, nout, grad);
+    k_reduce_parts<<<(nout + 31) / 32, 256, 0, st>>>(part, nblk, nout, grad);
 }
 
-void loss(const float* out, const float* tgt, const float* msk, int64_t n, int W, float inv_msum, float* dout,
+void loss(const float* out, const float* tgt, const float* msk, int64_t n, int W, float* dout,
           __nv_bfloat16* dpk, double* part, int nblk, double* total, cudaStream_t st) {
-    k_loss<<<nblk, 256, 0, st>>>(out, tgt, msk, n, W, inv_msum, dout, dpk, part);
-    k_sum_double<<<1, 32, 0, st>>>(part, nblk, total);
+    k_mask_sum<<<nblk, 256, 0, st>>>(msk, n, part + nblk);
+    k_loss<<<nblk, 256, 0, st>>>(out, tgt, msk, n, W, dout, dpk, part);
+    k_totals<<<1, 256, 0, st>>>(part, nblk, total);
 }
 
 void adam(float* w, float* m, float* v, const float* g, int n, float lr, float b1, float b2, float eps, float c1, float c2,

@@ -22,8 +22,9 @@ enum WgradKind { WGRAD_IN, WGRAD_MID, WGRAD_OUT };
 // Activations are BF16 in a channel-blocked layout [B][H][C / 8][W][8]: each 8-channel chunk of
 // an image row is W x 16 contiguous bytes.
 // TMA map of an activation (C % 8 == 0): boxes of one row, every chunk, 130 pixels (convolution
-// input: one halo pixel each side) or 128 pixels (weight-gradient operand); false when the
-// driver has no encoder or refuses the map.
+// input: one halo pixel each side) or 128 pixels (weight-gradient operand, as 256 elements of 8 bytes: a
+// chunk's pixels are one line of the box, not 128 of 16 bytes, which took a weight gradient of 1 M pixels
+// from 98 to 77 us); false when the driver has no encoder or refuses the map.
 bool encode_act_map(unsigned char out[128], const __nv_bfloat16* base, int C, int B, int H, int W, bool conv_box);
 
 void pack_input(const float* feat, __nv_bfloat16* x, int B, int H, int W, cudaStream_t st);
@@ -36,8 +37,8 @@ void conv(ConvKind kind, const void* in_map, const __nv_bfloat16* w, const float
 void wgrad(WgradKind kind, const void* x_map, const void* d_map, float* part, int max_blocks, float* grad, int B, int H,
            int W, unsigned int* err, uint64_t wait_ns, cudaStream_t st);
 // masked MSE: dout (FP32) and its packed BF16 form dpk (16 channels, blocked) = (dh, dl, dh, 0 ...);
-// the loss sum in *total
-void loss(const float* out, const float* tgt, const float* msk, int64_t n, int W, float inv_msum, float* dout,
+// the loss sum and the mask sum in total[0], total[1]; part: 2 nblk partials
+void loss(const float* out, const float* tgt, const float* msk, int64_t n, int W, float* dout,
           __nv_bfloat16* dpk, double* part, int nblk, double* total, cudaStream_t st);
 void adam(float* w, float* m, float* v, const float* g, int n, float lr, float b1, float b2, float eps, float c1, float c2,
           cudaStream_t st);

@@ -173,15 +173,8 @@ tomo_status backward(tomo_net* n, const float* feat, const float* tgt, const flo
                      double* loss_out) {
     cudaStream_t st = n->st;
     const int64_t P = (int64_t)B * H * W;
-    // mask sum on the host (the mask is a small input)
-    std::vector<float> hm(P);
-    NCU(n, cudaMemcpyAsync(hm.data(), msk, sizeof(float) * P, cudaMemcpyDeviceToHost, st));
-    NCU(n, cudaStreamSynchronize(st));
-    double ms = 0.0;
-    for (float x : hm) ms += x;
-    if (!(ms > 0.0)) return n->fail(TOMO_ERR_ARG, "mask is empty");
     forward(n, feat, B, H, W, n->out, st);
-    cnn::loss(n->out, tgt, msk, P, W, (float)(1.0 / ms), n->dout, n->dpk, n->lpart, kPartBlocks, n->ltot, st);
+    cnn::loss(n->out, tgt, msk, P, W, n->dout, n->dpk, n->lpart, kPartBlocks, n->ltot, st);
     // layer 5: weight gradient from the packed loss gradient, then the data gradient into layer 4
     cnn::wgrad(cnn::WGRAD_OUT, n->wmap[tomo_net::M_Y3], n->wmap[tomo_net::M_DPK], n->part, kPartBlocks, n->g + oW5, B,
                H, W, n->errd, n->wait_ns, st);
@@ -199,12 +192,13 @@ tomo_status backward(tomo_net* n, const float* feat, const float* tgt, const flo
     }
     cnn::wgrad(cnn::WGRAD_IN, n->wmap[tomo_net::M_X0], n->wmap[tomo_net::M_DZ0 + cur], n->part, kPartBlocks, n->g + oW1,
                B, H, W, n->errd, n->wait_ns, st);
-    double l = 0.0;
-    NCU(n, cudaMemcpyAsync(&l, n->ltot, sizeof(double), cudaMemcpyDeviceToHost, st));
+    double tot[2] = {0.0, 0.0};   // loss sum, mask sum (an empty mask's gradients are not finite and not used)
+    NCU(n, cudaMemcpyAsync(tot, n->ltot, sizeof tot, cudaMemcpyDeviceToHost, st));
     NCU(n, cudaStreamSynchronize(st));
     NCU(n, cudaGetLastError());
     if (tomo_status w = check_waits(n); w != TOMO_OK) return w;
-    if (loss_out) *loss_out = l / ms;
+    if (!(tot[1] > 0.0)) return n->fail(TOMO_ERR_ARG, "mask is empty");
+    if (loss_out) *loss_out = tot[0] / tot[1];
     return TOMO_OK;
 }
 
@@ -242,8 +236,8 @@ tomo_status tomo_net_create(int32_t device, uint64_t seed, tomo_net** out) try {
               n->alloc(&n->v, kParams) && n->alloc(&n->wf1, kW1);
     for (int l = 0; l < 3; ++l) ok = ok && n->alloc(&n->wf[l], kWmid) && n->alloc(&n->wd[l], kWmid);
     ok = ok && n->alloc(&n->wo, 9 * 16 * C) && n->alloc(&n->wod, 9 * 16 * C);
-    ok = ok && n->alloc(&n->part, (int64_t)kPartBlocks * (kWmid + C)) && n->alloc(&n->lpart, kPartBlocks) &&
-         n->alloc(&n->ltot, 1);
+    ok = ok && n->alloc(&n->part, (int64_t)kPartBlocks * (kWmid + C)) && n->alloc(&n->lpart, 2 * kPartBlocks) &&
+         n->alloc(&n->ltot, 2);
     if (!ok) return TOMO_ERR_OOM;
     if (cudaHostAlloc((void**)&n->errh, sizeof(unsigned int), cudaHostAllocMapped) != cudaSuccess) {
         n->errh = nullptr;

@@ -29,8 +29,8 @@
 // (dout = dh + dl) as a 16-channel input.  Both keep the FP32 layer's accuracy.
 //
 // Weight gradient (k_wgrad_tc): dW[tap][ci][co] = sum_p x[p + off(tap)][ci] dz[p][co]
-// with K = pixels, both operands MN-major.  Each input row arrives as three copies shifted by
-// one pixel, plus a constant plane of ones whose products give the bias gradient; accumulators
+// with K = pixels, both operands MN-major.  Each output-gradient row arrives as three copies shifted by
+// one pixel, each input row once, beside a constant plane of ones whose products give the bias gradient; accumulators
 // stay in TMEM over all the block's rows; each block writes one partial sum, reduced later in
 // fixed order, so training steps are deterministic.
 //
@@ -283,24 +283,30 @@ struct WgradArgs {
     uint64_t wait_ns;
 };
 
-// Row-streaming weight gradient.  Input row j of a strip lands in a ring slot as three copies
-// shifted by dx = 0, 1, 2 pixels (3 x CIN / 8 planes of 128 pixels x 16 B) plus a plane of
-// ones; slots 0 and 1 are mirrored after the last slot, so for any output row the three input
-// rows y - 1, y, y + 1 are consecutive slots and the planes (dy, dx, chunk) sit one plane apart:
-// the MMA's A operand rows are (tap, ci) at a uniform stride, with no im2col copy.
+// Row-streaming weight gradient.  Input row j of a strip lands in a ring slot as CIN / 8 planes of 128
+// pixels x 16 B, followed by a plane of ones; slots 0 and 1 are mirrored after the last slot, so for any
+// output row the three input rows y - 1, y, y + 1 are consecutive slots and the planes (dy, chunk) sit one
+// plane apart: the MMA's A operand rows are (dy, ci) at a uniform stride.  The output-gradient row lands as
+// three copies shifted by 1 - dx pixels, whose columns (dx, co) are its B operand, so one accumulator
+// of 128 x 96 takes all nine taps in 8 MMAs per row.  An MMA takes 64 cycles up to N = 64 at least, whatever N is:
+// with three groups of (tap, ci) rows and N = 32 it was 24 per row, and the three copies of the wider
+// operand left room for 5 input and 2 gradient rows in flight instead of 8 and 4.  Measured, 32 -> 32 channels,
+// 1 M pixels: 77 -> 42 us; the two operands' bytes take 20.
 template <int CIN, int NB>
 struct WgradShape {
     static constexpr int NCHX = CIN / 8;
-    static constexpr int NPL = 3 * NCHX + 1;                  // planes per input-row slot (ones last)
-    static constexpr int MG = (3 * NPL * 8 + 127) / 128;      // M groups of 128 rows (16 planes)
-    static constexpr int R = CIN == 32 ? 5 : 8;               // input row slots
-    static constexpr int XSLOTS = ((R - 1) * NPL + MG * 16 - 1) / NPL + 1;   // + mirrors and read slack
-    static constexpr int RD = CIN == 32 ? 2 : 4;              // output-gradient row slots
+    static constexpr int NPL = NCHX + 1;                      // planes per input-row slot (ones last)
+    static constexpr int MPL = 16;                            // planes of the A operand (3 NPL used)
+    static constexpr int N = 3 * NB;                          // B columns (dx, co)
+    static constexpr int R = 8;                               // input row slots
+    static constexpr int XSLOTS = ((R - 1) * NPL + MPL - 1) / NPL + 1;   // + mirrors and read slack
+    static constexpr int RD = 4;                              // output-gradient row slots
     static constexpr int XBYTES = XSLOTS * NPL * PLANE;
-    static constexpr int DSLOT = NB / 8 * PLANE;
-    static constexpr uint32_t NCOL = MG * NB <= 32 ? 32 : MG * NB <= 64 ? 64 : MG * NB <= 128 ? 128 : 256;
+    static constexpr int DCOPY = NB / 8 * PLANE, DSLOT = 3 * DCOPY;
+    static constexpr uint32_t NCOL = N <= 64 ? 64 : 128;
     static constexpr size_t SMEM = (size_t)XBYTES + (size_t)RD * DSLOT + (2 * R + 2 * RD + 1) * 8 + 16;
     static constexpr int NOUT = NB == 16 ? 9 * CIN + 1 : 9 * CIN * NB + NB;
+    static_assert(3 * NPL <= MPL && N % 16 == 0, "MMA tile");
     static_assert(XSLOTS >= R + 2, "mirror slots");
     static_assert(SMEM <= 232448, "shared memory");
 };
@@ -308,17 +314,17 @@ struct WgradShape {
 // NB = 32: part row = dW[tap][ci][co] (9 CIN 32 values) then db[co];
 // NB = 16 (output layer, dz = the packed loss gradient dh, dl): dW5[tap][ci] then db5, each the
 // sum of the dh and dl columns.  Roles as in k_conv_tc: warp 0 lane 0 loads, warp 1 lane 0 issues
-// the MMAs (3 M groups x 8 K steps per output row, accumulated over all the block's rows), warps
+// the MMAs (8 K steps per output row, accumulated over all the block's rows), warps
 // 2-5 read the accumulators at the end.
 template <int CIN, int NB>
 __global__ void __launch_bounds__(192, 1) k_wgrad_tc(const __grid_constant__ CUtensorMap x_map,
                                                     const __grid_constant__ CUtensorMap d_map, WgradArgs a, int RC) {
     using S = WgradShape<CIN, NB>;
-    constexpr int NCHX = S::NCHX, NPL = S::NPL, MG = S::MG, R = S::R, RD = S::RD;
-    constexpr uint32_t IDESC = idesc_bf16(128, NB, 1, 1);
+    constexpr int NCHX = S::NCHX, NPL = S::NPL, R = S::R, RD = S::RD;
+    constexpr uint32_t IDESC = idesc_bf16(128, S::N, 1, 1);
     extern __shared__ __align__(1024) unsigned char sm[];
     unsigned char* const xs = sm;                                            // [XSLOTS][NPL][PLANE]
-    unsigned char* const ds = sm + S::XBYTES;                                // [RD][NB / 8][PLANE]
+    unsigned char* const ds = sm + S::XBYTES;                                // [RD][3][NB / 8][PLANE]
     uint64_t* const xfull = reinterpret_cast<uint64_t*>(ds + RD * S::DSLOT); // [R]
     uint64_t* const xempty = xfull + R;
     uint64_t* const dfull = xempty + R;                                      // [RD]
@@ -347,7 +353,7 @@ __global__ void __launch_bounds__(192, 1) k_wgrad_tc(const __grid_constant__ CUt
     if (warp == 0) tmem_alloc(tslot, S::NCOL);
     // the ones plane of every slot (bias rows); TMA never writes it
     for (int sl = 0; sl < S::XSLOTS; ++sl) {
-        uint4* p = reinterpret_cast<uint4*>(xs + (sl * NPL + 3 * NCHX) * PLANE);
+        uint4* p = reinterpret_cast<uint4*>(xs + (sl * NPL + NCHX) * PLANE);
         for (int i = tid; i < PLANE / 16; i += blockDim.x) p[i] = make_uint4(0x3F803F80u, 0x3F803F80u, 0x3F803F80u, 0x3F803F80u);
     }
     fence_proxy_async();
@@ -372,12 +378,9 @@ __global__ void __launch_bounds__(192, 1) k_wgrad_tc(const __grid_constant__ CUt
                 const int s = q % R;
                 if (q >= R && !role_wait(&xempty[s], (uint32_t)(q / R - 1) & 1u, a.wait_ns, abort)) return false;
                 const int copies = s < 2 ? 2 : 1;   // slots 0 and 1 are mirrored at R and R + 1
-                mbar_expect_tx(&xfull[s], (uint32_t)(copies * 3 * NCHX * PLANE));
-                for (int m = 0; m < copies; ++m) {
-                    unsigned char* dst = xs + (m == 0 ? s : R + s) * NPL * PLANE;
-                    for (int dx = 0; dx < 3; ++dx)   // one box: every chunk of the row, shifted by dx
-                        tma_load_4d(dst + dx * NCHX * PLANE, &x_map, 2 * (x0 + dx - 1), 0, yy, b, &xfull[s]);
-                }
+                mbar_expect_tx(&xfull[s], (uint32_t)(copies * NCHX * PLANE));
+                for (int m = 0; m < copies; ++m)   // one box: every chunk of the row
+                    tma_load_4d(xs + (m == 0 ? s : R + s) * NPL * PLANE, &x_map, 2 * x0, 0, yy, b, &xfull[s]);
                 ++q;
                 return true;
             };
@@ -385,7 +388,8 @@ __global__ void __launch_bounds__(192, 1) k_wgrad_tc(const __grid_constant__ CUt
                 const int s = qd % RD;
                 if (qd >= RD && !role_wait(&dempty[s], (uint32_t)(qd / RD - 1) & 1u, a.wait_ns, abort)) return false;
                 mbar_expect_tx(&dfull[s], (uint32_t)S::DSLOT);
-                tma_load_4d(ds + s * S::DSLOT, &d_map, 2 * x0, 0, yy, b, &dfull[s]);
+                for (int dx = 0; dx < 3; ++dx)   // zero beyond the image: no tap reaches there
+                    tma_load_4d(ds + s * S::DSLOT + dx * S::DCOPY, &d_map, 2 * (x0 + 1 - dx), 0, yy, b, &dfull[s]);
                 ++qd;
                 return true;
             };
@@ -422,12 +426,8 @@ __global__ void __launch_bounds__(192, 1) k_wgrad_tc(const __grid_constant__ CUt
                     const uint64_t xd = xdesc0 + (uint64_t)(((qb + k) % R) * (NPL * PLANE / 16));
                     const uint64_t dd = ddesc0 + (uint64_t)((t % RD) * (S::DSLOT / 16));
 #pragma unroll
-                    for (int g = 0; g < MG; ++g) {
-#pragma unroll
-                        for (int kk = 0; kk < TX / 16; ++kk)
-                            umma_bf16(tmem + g * NB, xd + (uint64_t)((g * 16 * PLANE + kk * 256) / 16),
-                                      dd + (uint64_t)(kk * 256 / 16), IDESC, (t | kk) != 0);
-                    }
+                    for (int kk = 0; kk < TX / 16; ++kk)
+                        umma_bf16(tmem, xd + (uint64_t)(kk * 256 / 16), dd + (uint64_t)(kk * 256 / 16), IDESC, (t | kk) != 0);
                     umma_commit(&dempty[t % RD]);
                     umma_commit(&xempty[(qb + k) % R]);
                 }
@@ -448,21 +448,22 @@ __global__ void __launch_bounds__(192, 1) k_wgrad_tc(const __grid_constant__ CUt
     if (ok && warp >= 2) {
         const int quarter = warp & 3;
         float* const out = a.part + (int64_t)blockIdx.x * S::NOUT;
+        const int m = 32 * quarter + lane, p = m / 8, i = m % 8;   // window row: plane, channel in it
+        const int dy = p / NPL, rem = p % NPL;
 #pragma unroll
-        for (int g = 0; g < MG; ++g) {
+        for (int dx = 0; dx < 3; ++dx) {
             float v[NB];
-            const uint32_t taddr = tmem + ((uint32_t)(32 * quarter) << 16) + (uint32_t)(g * NB);
+            __syncwarp();
+            const uint32_t taddr = tmem + ((uint32_t)(32 * quarter) << 16) + (uint32_t)(dx * NB);
             if constexpr (NB == 32) tmem_ld32(taddr, v);
             else tmem_ld16(taddr, v);
             if (!any) {
 #pragma unroll
                 for (int n = 0; n < NB; ++n) v[n] = 0.f;
             }
-            const int m = g * 128 + 32 * quarter + lane;   // window row: plane m / 8, channel m % 8
-            const int p = m / 8, i = m % 8, dy = p / NPL, rem = p % NPL;
             int row = -1;                                   // output row: tap * CIN + ci, or 9 CIN = bias
-            if (dy < 3 && rem < 3 * NCHX) row = (dy * 3 + rem / NCHX) * CIN + (rem % NCHX) * 8 + i;
-            else if (dy == 0 && rem == 3 * NCHX && i == 0) row = 9 * CIN;
+            if (dy < 3 && rem < NCHX) row = (dy * 3 + dx) * CIN + rem * 8 + i;
+            else if (dy == 0 && dx == 1 && i == 0) row = 9 * CIN;
             if (row < 0) continue;
             if constexpr (NB == 16) {
                 out[row] = v[0] + v[1];

@@ -7,9 +7,8 @@
 //   layer 5: 32 -> 1, bias, FP32 output (the proposed field update)
 //
 // Activations are BF16 in a channel-blocked layout, [image][y][channel / 8][x][8]: each
-// 8-channel chunk of an image row is contiguous, so one TMA box brings a whole input row (all
-// chunks, 130 pixels) into shared memory already in the tensor cores' K-major core-matrix
-// layout (8 pixels x 16 bytes).  Every convolution and every weight gradient runs on the
+// 8-channel chunk of an image row is contiguous, so TMA boxes bring input rows into shared memory
+// already in the tensor cores' K-major core-matrix layout (8 pixels x 16 bytes).  Every convolution and every weight gradient runs on the
 // fifth-generation tensor cores (tcgen05.mma, kind::f16, BF16 operands, FP32 accumulators in
 // tensor memory), in warp-specialised blocks: one thread issues the TMA copies, one the MMAs,
 // four warps drain the accumulators; barriers are mbarriers whose waits are bounded.
@@ -73,15 +72,16 @@ struct ConvArgs {
 };
 
 // Row-streaming convolution.  A work item is a strip of up to RC output rows of one 128-pixel
-// column tile of one image; each of its RC + 2 input rows arrives as one TMA box (every
-// 8-channel chunk, 130 pixels: one halo pixel each side) into a ring of R row slots.
+// column tile of one image; each of its RC + 2 input rows arrives, chunk by chunk, as a TMA box of 128
+// pixels and one of the 2 that remain (one halo pixel each side; elements of 8 bytes, at most 256 to a line)
+// into a ring of R row slots.
 template <int CIN, int N>
 struct ConvShape {
     static constexpr int NCH = CIN / 8;                        // input chunks
-    static constexpr int CP = PX * 16;                         // bytes per chunk row: 130 pixels x 16 B
+    static constexpr int CP = (PX * 16 + 127) / 128 * 128;     // bytes per chunk row: 130 pixels x 16 B, padded
     static constexpr int R = 8;                                // input row slots
-    static constexpr int NA = 4;                               // TMEM accumulators (output rows in flight)
-    static constexpr int SLOT = (NCH * CP + 127) / 128 * 128;  // one input row, all chunks (one TMA box)
+    static constexpr int NA = 8;                               // TMEM accumulators (output rows in flight)
+    static constexpr int SLOT = NCH * CP;                      // one input row, all chunks
     static constexpr int WBYTES = 9 * NCH * N * 16;            // weights
     static constexpr uint32_t ROW_BYTES = (uint32_t)NCH * PX * 16;
     static constexpr uint32_t NCOL = NA * N < 32 ? 32 : NA * N;
@@ -90,19 +90,22 @@ struct ConvShape {
 };
 
 // Warp roles (192 threads): warp 0 lane 0 issues the TMA row loads, warp 1 lane 0 issues the
-// MMAs (9 taps x CIN / 16 per output row into one of NA accumulators; the A operand of tap
-// (dy, dx) is row slot (k + dy) moved by dx pixels), warps 2-5 drain the accumulators (their
-// TMEM lane quarters are warp % 4) and store.  Barriers: full / empty per row slot (TMA
-// transaction bytes / MMA commit once the slot's last reader has run), full / empty per
-// accumulator (MMA commit / one arrival per epilogue warp).
+// MMAs (3 dx x CIN / 16 per input row; the A operand is the row's slot moved by dx pixels, the B
+// operand the weights of dy = 2, 1, 0, and the 3 N columns the neighbouring accumulators of the output rows
+// j - 2, j - 1, j), warps 2-5 drain the accumulators (their TMEM lane quarters are warp % 4) and store.
+// A row takes 7 or 8 MMAs of up to 96 columns where one per tap and 16 channels takes 18 of 32, and its slot is
+// free after them, not two rows later; 32 -> 32 channels, 512 x 512: 27.0 -> 24.5 us cold, 1 M pixels 40.9 -> 38
+// (the bytes take 20; at about 1300 multiply-adds per cycle and SM the tensor core is what the rows wait
+// for).  An accumulator's products come in the order (dy, dx, channels), as one MMA per tap gives them: same bits.  Barriers: full / empty per row slot (TMA transaction bytes /
+// MMA commit), full / empty per accumulator (MMA commit of its last input row / one arrival per epilogue warp).
 template <int CIN, int N, int EPI>
-__global__ void __launch_bounds__(192, 2) k_conv_tc(const __grid_constant__ CUtensorMap in_map, ConvArgs a, int RC) {
+__global__ void __launch_bounds__(192, 2) k_conv_tc(const __grid_constant__ CUtensorMap line_map, const __grid_constant__ CUtensorMap halo_map,
+                                                    ConvArgs a, int RC) {
     using S = ConvShape<CIN, N>;
     constexpr int NCH = S::NCH, KS = CIN / 16, R = S::R, NA = S::NA;
-    constexpr uint32_t IDESC = idesc_bf16(128, N, 0, 0);
     extern __shared__ __align__(1024) unsigned char sm[];
     unsigned char* const rows = sm;                                          // [R][NCH][CP]
-    unsigned char* const wsm = sm + R * S::SLOT;                             // [9][NCH][N][16 B]
+    unsigned char* const wsm = sm + R * S::SLOT;                             // [dx][NCH][2 - dy][N][16 B]
     uint64_t* const full = reinterpret_cast<uint64_t*>(wsm + S::WBYTES);     // [R]
     uint64_t* const empty = full + R;                                        // [R]
     uint64_t* const accf = empty + R;                                        // [NA]
@@ -130,8 +133,10 @@ __global__ void __launch_bounds__(192, 2) k_conv_tc(const __grid_constant__ CUte
     }
     __syncwarp();
     if (warp == 0) tmem_alloc(tslot, S::NCOL);
-    for (int i = tid; i < S::WBYTES / 16; i += blockDim.x)
-        reinterpret_cast<uint4*>(wsm)[i] = reinterpret_cast<const uint4*>(a.w)[i];
+    for (int i = tid; i < S::WBYTES / 16; i += blockDim.x) {   // from [dy][dx][NCH][N]
+        const int n = i % N, q = i / N % NCH, dx = i / (N * NCH) % 3, dy = i / (3 * N * NCH);
+        reinterpret_cast<uint4*>(wsm)[((dx * NCH + q) * 3 + 2 - dy) * N + n] = reinterpret_cast<const uint4*>(a.w)[i];
+    }
     if (EPI == EPI_RELU && tid < N) sbias[tid] = a.bias[tid];
     if (EPI == EPI_OUT && tid == 0) sbias[0] = a.bias[0];
     fence_proxy_async();
@@ -163,7 +168,11 @@ __global__ void __launch_bounds__(192, 2) k_conv_tc(const __grid_constant__ CUte
                         break;
                     }
                     mbar_expect_tx(&full[s], S::ROW_BYTES);
-                    tma_load_5d(rows + s * S::SLOT, &in_map, 0, x0 - 1, 0, y0 - 1 + j, b, &full[s]);
+                    for (int c = 0; c < NCH; ++c) {
+                        unsigned char* const dst = rows + s * S::SLOT + c * S::CP;
+                        tma_load_4d(dst, &line_map, 2 * (x0 - 1), c, y0 - 1 + j, b, &full[s]);
+                        tma_load_4d(dst + TX * 16, &halo_map, 2 * (x0 + TX - 1), c, y0 - 1 + j, b, &full[s]);
+                    }
                 }
             }
             // no copy may land after the block has left: wait (bounded) for the last use of each slot
@@ -171,43 +180,49 @@ __global__ void __launch_bounds__(192, 2) k_conv_tc(const __grid_constant__ CUte
         }
     } else if (warp == 1) {
         if (lane == 0) {   // MMA issuer
-            int qb = 0, t = 0;
+            int q = 0, t0 = 0;   // input rows and output rows before this item
             bool ok = true;
-            const uint64_t adesc0 = smem_desc(sm_addr(rows), S::CP, 128);   // row slot 0, chunk 0, pixel 0
-            const uint64_t bdesc0 = smem_desc(sm_addr(wsm), N * 16, 128);   // tap 0, chunk 0
+            const uint64_t adesc0 = smem_desc(sm_addr(rows), S::CP, 128);       // row slot 0, chunk 0, pixel 0
+            const uint64_t bdesc0 = smem_desc(sm_addr(wsm), 3 * N * 16, 128);   // dx 0, chunk 0, dy 2
             for (int it = blockIdx.x; it < items && ok; it += gridDim.x) {
                 int b, x0, y0, n;
                 item_at(it, b, x0, y0, n);
-                for (int k = 0; k < n; ++k, ++t) {
-                    for (int r = k == 0 ? 0 : 2; r < 3 && ok; ++r) {
-                        const int qq = qb + k + r;
-                        ok = role_wait(&full[qq % R], (uint32_t)(qq / R) & 1u, a.wait_ns, abort);
-                    }
-                    const int acc = t % NA;
-                    if (ok && t >= NA) ok = role_wait(&acce[acc], (uint32_t)(t / NA - 1) & 1u, a.wait_ns, abort);
+                for (int j = 0; j < n + 2; ++j, ++q) {   // input row j reaches output rows k = j - dy
+                    const int klo = max(j - 2, 0), khi = min(j, n - 1);
+                    ok = role_wait(&full[q % R], (uint32_t)(q / R) & 1u, a.wait_ns, abort);
+                    const int tn = t0 + j;               // output row j begins
+                    if (ok && j < n && tn >= NA) ok = role_wait(&acce[tn % NA], (uint32_t)(tn / NA - 1) & 1u, a.wait_ns, abort);
                     if (!ok) break;
                     tc_fence_after();
                     // descriptors: the start-address field is the low 14 bits (address / 16), so a
                     // byte offset o below 256 KB is added as o / 16
-                    uint64_t arow[3];
+                    const uint64_t arow = adesc0 + (uint64_t)((q % R) * (S::SLOT / 16));
+                    // MMAs of the output rows k .. ke, up to the end of the accumulator ring at a time
+                    auto mma = [&](uint64_t ad, uint64_t bd, int k, int ke, uint32_t accumulate) {
+                        while (k <= ke) {
+                            const int at = (t0 + k) % NA, cnt = min(ke - k + 1, NA - at);
+                            umma_bf16(tmem + at * N, ad, bd + (uint64_t)((k - j + 2) * N), idesc_bf16(128, cnt * N, 0, 0), accumulate);
+                            k += cnt;
+                        }
+                    };
 #pragma unroll
-                    for (int dy = 0; dy < 3; ++dy) arow[dy] = adesc0 + (uint64_t)(((qb + k + dy) % R) * (S::SLOT / 16));
-#pragma unroll
-                    for (int tap = 0; tap < 9; ++tap) {
+                    for (int dx = 0; dx < 3; ++dx) {
 #pragma unroll
                         for (int ks = 0; ks < KS; ++ks) {
-                            const uint64_t ad = arow[tap / 3] + (uint64_t)(((tap % 3) * 16 + 2 * ks * S::CP) / 16);
-                            const uint64_t bd = bdesc0 + (uint64_t)((tap * NCH + 2 * ks) * N);
-                            umma_bf16(tmem + acc * N, ad, bd, IDESC, (tap | ks) != 0);
+                            const uint64_t ad = arow + (uint64_t)((dx * 16 + 2 * ks * S::CP) / 16);
+                            const uint64_t bd = bdesc0 + (uint64_t)((dx * NCH + 2 * ks) * 3 * N);
+                            if (dx == 0 && ks == 0 && khi == j) {   // the first product of row j starts its accumulator
+                                mma(ad, bd, klo, j - 1, 1u);
+                                mma(ad, bd, j, j, 0u);
+                            } else {
+                                mma(ad, bd, klo, khi, 1u);
+                            }
                         }
                     }
-                    umma_commit(&accf[acc]);
-                    umma_commit(&empty[(qb + k) % R]);   // input row k has had its last reader
+                    umma_commit(&empty[q % R]);
+                    if (j >= 2) umma_commit(&accf[(t0 + j - 2) % NA]);
                 }
-                if (!ok) break;
-                umma_commit(&empty[(qb + n) % R]);
-                umma_commit(&empty[(qb + n + 1) % R]);
-                qb += n + 2;
+                t0 += n;
             }
             // every MMA this thread issued has completed once `done` flips
             umma_commit(done);
@@ -288,9 +303,9 @@ struct WgradArgs {
 // output row the three input rows y - 1, y, y + 1 are consecutive slots and the planes (dy, chunk) sit one
 // plane apart: the MMA's A operand rows are (dy, ci) at a uniform stride.  The output-gradient row lands as
 // three copies shifted by 1 - dx pixels, whose columns (dx, co) are its B operand, so one accumulator
-// of 128 x 96 takes all nine taps in 8 MMAs per row.  An MMA takes 64 cycles up to N = 64 at least, whatever N is:
-// with three groups of (tap, ci) rows and N = 32 it was 24 per row, and the three copies of the wider
-// operand left room for 5 input and 2 gradient rows in flight instead of 8 and 4.  Measured, 32 -> 32 channels,
+// of 128 x 96 takes all nine taps in 8 MMAs per row.  With the copies on the input's side, three groups of (tap,
+// ci) rows and N = 32, it was 24 per row, and the copies of the wider operand left room for 5 input and 2
+// gradient rows in flight instead of 8 and 4.  Measured, 32 -> 32 channels,
 // 1 M pixels: 77 -> 42 us; the two operands' bytes take 20.
 template <int CIN, int NB>
 struct WgradShape {
@@ -637,7 +652,7 @@ int sm_count() {
 }
 
 template <int CIN, int N, int EPI>
-void conv_launch(const void* map, const ConvArgs& a, cudaStream_t st) {
+void conv_launch(const ActMaps& in, const ConvArgs& a, cudaStream_t st) {
     using S = ConvShape<CIN, N>;
     auto kern = k_conv_tc<CIN, N, EPI>;
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM);
@@ -650,9 +665,10 @@ void conv_launch(const void* map, const ConvArgs& a, cudaStream_t st) {
     const int RC = (int)std::max<int64_t>(2, (a.H + strips - 1) / strips);
     const int64_t items = columns * ((a.H + RC - 1) / RC);
     const int grid = (int)std::max<int64_t>(1, std::min(items, slots));
-    CUtensorMap m;
-    std::memcpy(&m, map, sizeof m);
-    kern<<<grid, 192, S::SMEM, st>>>(m, a, RC);
+    CUtensorMap line, halo;
+    std::memcpy(&line, in.line, sizeof line);
+    std::memcpy(&halo, in.halo, sizeof halo);
+    kern<<<grid, 192, S::SMEM, st>>>(line, halo, a, RC);
 }
 
 template <int CIN, int NB>
@@ -682,30 +698,19 @@ using EncodeTiled = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, 
 }  // namespace
 
 // ---- tensor maps ------------------------------------------------------------------
-bool encode_act_map(unsigned char out[128], const __nv_bfloat16* base, int C, int B, int H, int W, bool conv_box) {
+bool encode_act_map(unsigned char out[128], const __nv_bfloat16* base, int C, int B, int H, int W, ActBox which) {
     const EncodeTiled fn = reinterpret_cast<EncodeTiled>(tensor_map_encoder());
     if (!fn || C % 8 != 0) return false;
     CUtensorMap m;
+    // blocked layout [b][y][C / 8][x][8] as elements of 8 bytes: dimensions (half pixel, chunk, y, image)
     const cuuint64_t nch = (cuuint64_t)C / 8;
-    CUresult r;
-    if (conv_box) {
-        // blocked layout [b][y][C / 8][x][8]: dimensions (channel in chunk, x, chunk, y, image)
-        const cuuint64_t dims[5] = {8u, (cuuint64_t)W, nch, (cuuint64_t)H, (cuuint64_t)B};
-        const cuuint64_t strides[4] = {16u, (cuuint64_t)W * 16u, nch * W * 16u, (cuuint64_t)H * nch * W * 16u};
-        const cuuint32_t box[5] = {8u, (cuuint32_t)PX, (cuuint32_t)nch, 1u, 1u};
-        const cuuint32_t estr[5] = {1u, 1u, 1u, 1u, 1u};
-        r = fn(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5u, const_cast<__nv_bfloat16*>(base), dims, strides, box, estr,
-               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    } else {
-        const cuuint64_t dims[4] = {2 * (cuuint64_t)W, nch, (cuuint64_t)H, (cuuint64_t)B};
-        const cuuint64_t strides[3] = {(cuuint64_t)W * 16u, nch * W * 16u, (cuuint64_t)H * nch * W * 16u};
-        const cuuint32_t box[4] = {2u * TX, (cuuint32_t)nch, 1u, 1u};
-        const cuuint32_t estr[4] = {1u, 1u, 1u, 1u};
-        r = fn(&m, CU_TENSOR_MAP_DATA_TYPE_UINT64, 4u, const_cast<__nv_bfloat16*>(base), dims, strides, box, estr,
-               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    }
+    const cuuint64_t dims[4] = {2 * (cuuint64_t)W, nch, (cuuint64_t)H, (cuuint64_t)B};
+    const cuuint64_t strides[3] = {(cuuint64_t)W * 16u, nch * W * 16u, (cuuint64_t)H * nch * W * 16u};
+    const cuuint32_t box[4] = {2u * (which == BOX_HALO ? PX - TX : TX), which == BOX_ROW ? (cuuint32_t)nch : 1u, 1u, 1u};
+    const cuuint32_t estr[4] = {1u, 1u, 1u, 1u};
+    const CUresult r = fn(&m, CU_TENSOR_MAP_DATA_TYPE_UINT64, 4u, const_cast<__nv_bfloat16*>(base), dims, strides, box, estr,
+                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return false;
     std::memcpy(out, &m, sizeof m);
     return true;
@@ -716,33 +721,33 @@ void pack_input(const float* feat, __nv_bfloat16* x, int B, int H, int W, cudaSt
     k_pack_input<<<blocks_for((int64_t)B * H * W, 256), 256, 0, st>>>(feat, x, B, H, W);
 }
 
-void conv(ConvKind kind, const void* in_map, const __nv_bfloat16* w, const float* bias, const __nv_bfloat16* mask,
+void conv(ConvKind kind, const ActMaps& in, const __nv_bfloat16* w, const float* bias, const __nv_bfloat16* mask,
           void* out, int B, int H, int W, unsigned int* err, uint64_t wait_ns, cudaStream_t st) {
     const ConvArgs a{w, bias, mask, out, B, H, W, err, wait_ns};
     switch (kind) {
-    case CONV_IN: conv_launch<16, 32, EPI_RELU>(in_map, a, st); break;
-    case CONV_MID: conv_launch<32, 32, EPI_RELU>(in_map, a, st); break;
-    case CONV_DGRAD: conv_launch<32, 32, EPI_MASK>(in_map, a, st); break;
-    case CONV_OUT: conv_launch<32, 16, EPI_OUT>(in_map, a, st); break;
-    case CONV_OUT_DGRAD: conv_launch<16, 32, EPI_MASK>(in_map, a, st); break;
+    case CONV_IN: conv_launch<16, 32, EPI_RELU>(in, a, st); break;
+    case CONV_MID: conv_launch<32, 32, EPI_RELU>(in, a, st); break;
+    case CONV_DGRAD: conv_launch<32, 32, EPI_MASK>(in, a, st); break;
+    case CONV_OUT: conv_launch<32, 16, EPI_OUT>(in, a, st); break;
+    case CONV_OUT_DGRAD: conv_launch<16, 32, EPI_MASK>(in, a, st); break;
     }
 }
 
-void wgrad(WgradKind kind, const void* x_map, const void* d_map, float* part, int max_blocks, float* grad, int B, int H,
+void wgrad(WgradKind kind, const ActMaps& x, const ActMaps& d, float* part, int max_blocks, float* grad, int B, int H,
            int W, unsigned int* err, uint64_t wait_ns, cudaStream_t st) {
     const WgradArgs a{part, B, H, W, err, wait_ns};
     int nblk = 1, nout = 1;
     switch (kind) {
     case WGRAD_IN:
-        nblk = wgrad_launch<16, 32>(x_map, d_map, a, max_blocks, st);
+        nblk = wgrad_launch<16, 32>(x.row, d.row, a, max_blocks, st);
         nout = WgradShape<16, 32>::NOUT;
         break;
     case WGRAD_MID:
-        nblk = wgrad_launch<32, 32>(x_map, d_map, a, max_blocks, st);
+        nblk = wgrad_launch<32, 32>(x.row, d.row, a, max_blocks, st);
         nout = WgradShape<32, 32>::NOUT;
         break;
     case WGRAD_OUT:
-        nblk = wgrad_launch<32, 16>(x_map, d_map, a, max_blocks, st);
+        nblk = wgrad_launch<32, 16>(x.row, d.row, a, max_blocks, st);
         nout = WgradShape<32, 16>::NOUT;
         break;
     }

@@ -21,20 +21,24 @@ enum WgradKind { WGRAD_IN, WGRAD_MID, WGRAD_OUT };
 
 // Activations are BF16 in a channel-blocked layout [B][H][C / 8][W][8]: each 8-channel chunk of
 // an image row is W x 16 contiguous bytes.
-// TMA map of an activation (C % 8 == 0): boxes of one row, every chunk, 130 pixels (convolution
-// input: one halo pixel each side) or 128 pixels (weight-gradient operand, as 256 elements of 8 bytes: a
-// chunk's pixels are one line of the box, not 128 of 16 bytes, which took a weight gradient of 1 M pixels
-// from 98 to 77 us); false when the driver has no encoder or refuses the map.
-bool encode_act_map(unsigned char out[128], const __nv_bfloat16* base, int C, int B, int H, int W, bool conv_box);
+// TMA maps of an activation (C % 8 == 0), in elements of 8 bytes, so that a chunk's pixels are one line of a
+// box and not 128 of 16 bytes (which took a weight gradient of 1 M pixels from 98 to 77 us).  Boxes: 128
+// pixels of every chunk of a row (weight-gradient operands), 128 and 2 pixels of one chunk (convolution input,
+// one halo pixel each side).  encode_act_map: false when the driver has no encoder or refuses the map.
+enum ActBox { BOX_ROW, BOX_LINE, BOX_HALO };
+struct ActMaps {
+    alignas(64) unsigned char row[128], line[128], halo[128];
+};
+bool encode_act_map(unsigned char out[128], const __nv_bfloat16* base, int C, int B, int H, int W, ActBox which);
 
 void pack_input(const float* feat, __nv_bfloat16* x, int B, int H, int W, cudaStream_t st);
 // out = conv(in) with the packed weights w (pack_weights / pack_out_weights layouts); a timed-out
 // wait sets bit 1 of *err (host-visible).
-void conv(ConvKind kind, const void* in_map, const __nv_bfloat16* w, const float* bias, const __nv_bfloat16* mask,
+void conv(ConvKind kind, const ActMaps& in, const __nv_bfloat16* w, const float* bias, const __nv_bfloat16* mask,
           void* out, int B, int H, int W, unsigned int* err, uint64_t wait_ns, cudaStream_t st);
-// grad = weight and bias gradient of a layer from its input (x_map) and output gradient (d_map),
+// grad = weight and bias gradient of a layer from its input x and output gradient d,
 // through per-block partials in part (at most max_blocks rows) reduced in fixed order.
-void wgrad(WgradKind kind, const void* x_map, const void* d_map, float* part, int max_blocks, float* grad, int B, int H,
+void wgrad(WgradKind kind, const ActMaps& x, const ActMaps& d, float* part, int max_blocks, float* grad, int B, int H,
            int W, unsigned int* err, uint64_t wait_ns, cudaStream_t st);
 // masked MSE: dout (FP32) and its packed BF16 form dpk (16 channels, blocked) = (dh, dl, dh, 0 ...);
 // the loss sum and the mask sum in total[0], total[1]; part: 2 nblk partials

@@ -53,11 +53,9 @@ struct tomo_net {
     int64_t cap = 0;
     __nv_bfloat16 *x0 = nullptr, *y[4] = {}, *dz[2] = {}, *dpk = nullptr;
     float *out = nullptr, *dout = nullptr, *msk_sum = nullptr;
-    // TMA maps of the activations for shape (mB, mH, mW): convolution-input boxes and
-    // weight-gradient boxes
+    // TMA maps of the activations for shape (mB, mH, mW)
     enum { M_X0, M_Y0, M_Y1, M_Y2, M_Y3, M_DZ0, M_DZ1, M_DPK, NMAPS };
-    alignas(64) unsigned char cmap[NMAPS][128];
-    alignas(64) unsigned char wmap[NMAPS][128];
+    cnn::ActMaps maps[NMAPS];
     int mB = 0, mH = 0, mW = 0;
     int64_t step = 0;
     std::vector<void*> allocs;
@@ -135,8 +133,9 @@ tomo_status ensure_maps(tomo_net* n, int B, int H, int W) {
     const __nv_bfloat16* base[tomo_net::NMAPS] = {n->x0, n->y[0], n->y[1], n->y[2], n->y[3], n->dz[0], n->dz[1], n->dpk};
     const int ch[tomo_net::NMAPS] = {16, C, C, C, C, C, C, 16};
     for (int i = 0; i < tomo_net::NMAPS; ++i)
-        if (!cnn::encode_act_map(n->cmap[i], base[i], ch[i], B, H, W, true) ||
-            !cnn::encode_act_map(n->wmap[i], base[i], ch[i], B, H, W, false)) {
+        if (!cnn::encode_act_map(n->maps[i].row, base[i], ch[i], B, H, W, cnn::BOX_ROW) ||
+            !cnn::encode_act_map(n->maps[i].line, base[i], ch[i], B, H, W, cnn::BOX_LINE) ||
+            !cnn::encode_act_map(n->maps[i].halo, base[i], ch[i], B, H, W, cnn::BOX_HALO)) {
             n->mB = n->mH = n->mW = 0;
             return n->fail(TOMO_ERR_CUDA, "cuTensorMapEncodeTiled refused an activation map");
         }
@@ -161,11 +160,11 @@ tomo_status check_waits(tomo_net* n) {
 void forward(tomo_net* n, const float* feat, int B, int H, int W, float* out, cudaStream_t st) {
     cnn::pack_input(feat, n->x0, B, H, W, st);
     const float* bias[4] = {n->w + ob1, n->w + ob2, n->w + ob3, n->w + ob4};
-    cnn::conv(cnn::CONV_IN, n->cmap[tomo_net::M_X0], n->wf1, bias[0], nullptr, n->y[0], B, H, W, n->errd, n->wait_ns, st);
+    cnn::conv(cnn::CONV_IN, n->maps[tomo_net::M_X0], n->wf1, bias[0], nullptr, n->y[0], B, H, W, n->errd, n->wait_ns, st);
     for (int l = 0; l < 3; ++l)
-        cnn::conv(cnn::CONV_MID, n->cmap[tomo_net::M_Y0 + l], n->wf[l], bias[l + 1], nullptr, n->y[l + 1], B, H, W,
+        cnn::conv(cnn::CONV_MID, n->maps[tomo_net::M_Y0 + l], n->wf[l], bias[l + 1], nullptr, n->y[l + 1], B, H, W,
                   n->errd, n->wait_ns, st);
-    cnn::conv(cnn::CONV_OUT, n->cmap[tomo_net::M_Y3], n->wo, n->w + ob5, nullptr, out, B, H, W, n->errd, n->wait_ns, st);
+    cnn::conv(cnn::CONV_OUT, n->maps[tomo_net::M_Y3], n->wo, n->w + ob5, nullptr, out, B, H, W, n->errd, n->wait_ns, st);
 }
 
 // loss and gradient into n->g
@@ -176,21 +175,21 @@ tomo_status backward(tomo_net* n, const float* feat, const float* tgt, const flo
     forward(n, feat, B, H, W, n->out, st);
     cnn::loss(n->out, tgt, msk, P, W, n->dout, n->dpk, n->lpart, kPartBlocks, n->ltot, st);
     // layer 5: weight gradient from the packed loss gradient, then the data gradient into layer 4
-    cnn::wgrad(cnn::WGRAD_OUT, n->wmap[tomo_net::M_Y3], n->wmap[tomo_net::M_DPK], n->part, kPartBlocks, n->g + oW5, B,
+    cnn::wgrad(cnn::WGRAD_OUT, n->maps[tomo_net::M_Y3], n->maps[tomo_net::M_DPK], n->part, kPartBlocks, n->g + oW5, B,
                H, W, n->errd, n->wait_ns, st);
-    cnn::conv(cnn::CONV_OUT_DGRAD, n->cmap[tomo_net::M_DPK], n->wod, nullptr, n->y[3], n->dz[0], B, H, W, n->errd,
+    cnn::conv(cnn::CONV_OUT_DGRAD, n->maps[tomo_net::M_DPK], n->wod, nullptr, n->y[3], n->dz[0], B, H, W, n->errd,
               n->wait_ns, st);
     // layers 4, 3, 2: weight gradient, then data gradient masked by the layer input's ReLU
     const int64_t ow[3] = {oW2, oW3, oW4};
     int cur = 0;
     for (int l = 2; l >= 0; --l) {   // l = index of layers 2..4 in wf/wd; input activation y[l]
-        cnn::wgrad(cnn::WGRAD_MID, n->wmap[tomo_net::M_Y0 + l], n->wmap[tomo_net::M_DZ0 + cur], n->part, kPartBlocks,
+        cnn::wgrad(cnn::WGRAD_MID, n->maps[tomo_net::M_Y0 + l], n->maps[tomo_net::M_DZ0 + cur], n->part, kPartBlocks,
                    n->g + ow[l], B, H, W, n->errd, n->wait_ns, st);
-        cnn::conv(cnn::CONV_DGRAD, n->cmap[tomo_net::M_DZ0 + cur], n->wd[l], nullptr, n->y[l], n->dz[1 - cur], B, H, W,
+        cnn::conv(cnn::CONV_DGRAD, n->maps[tomo_net::M_DZ0 + cur], n->wd[l], nullptr, n->y[l], n->dz[1 - cur], B, H, W,
                   n->errd, n->wait_ns, st);
         cur = 1 - cur;
     }
-    cnn::wgrad(cnn::WGRAD_IN, n->wmap[tomo_net::M_X0], n->wmap[tomo_net::M_DZ0 + cur], n->part, kPartBlocks, n->g + oW1,
+    cnn::wgrad(cnn::WGRAD_IN, n->maps[tomo_net::M_X0], n->maps[tomo_net::M_DZ0 + cur], n->part, kPartBlocks, n->g + oW1,
                B, H, W, n->errd, n->wait_ns, st);
     double tot[2] = {0.0, 0.0};   // loss sum, mask sum (an empty mask's gradients are not finite and not used)
     NCU(n, cudaMemcpyAsync(tot, n->ltot, sizeof tot, cudaMemcpyDeviceToHost, st));

@@ -22,8 +22,8 @@ constexpr int kMaxCluster = 16;
 // z, the previous z, its products and the correlation, 4 x cells per thread, beside about 90 others,
 // so a block of up to 8 warps (255 registers) takes 32 cells per thread and one of up to 16 warps
 // (128 registers) 16.  A 512 x 512 grid would need 64 cells per thread on 16 blocks: tried, it
-// spills (41 us per adjoint step of 32 groups against 26 us in the strip kernels), so such grids stay
-// with the strip and tile kernels.
+// spills (41 us per adjoint step of 32 groups against 26 us in the strip kernels and 22 streamed), so such
+// grids are streamed or stay with the strip and tile kernels.
 int cells_per_lane(int nx) {
     for (const int c : {2, 4, 6, 8, 10, 12, 16})
         if (nx <= 32 * c) return c;

@@ -127,12 +127,12 @@ __global__ void __launch_bounds__(SW * 32, 4) k_stream_fwd(DevGeo g, StreamFwd a
     const int y0 = id / a.strips % a.bands * a.R, yend = min(y0 + a.R, ny);
     // per warp: u, v [FD][FW]; c [FC][FW]; receivers; sponge factor of each row
     constexpr int WF = (2 * FD + FC) * FW;
-    float* const base = reinterpret_cast<float*>(smem4) + w * (WF + 2 * MAXR + 16 + 2 * NREC);
+    float* const base = reinterpret_cast<float*>(smem4) + w * (WF + 2 * MAXR + 16 + NREC);
     float* const ru = base + 4 * lane;                     // this lane's places
     constexpr int V = FD * FW, C = 2 * FD * FW;            // from u: v, c
     RowRec* const rows = reinterpret_cast<RowRec*>(base + WF);
     int* const ent = reinterpret_cast<int*>(base + WF + MAXR);
-    float* const drow = base + WF + MAXR + 2 * NREC;       // of row ja + t
+    float* const drow = base + WF + MAXR + NREC;       // of row ja + t
     if (gl >= a.ng) return;
     const bool own = i >= 0 && i < g.nx && lane >= FH / 4 && lane < (FW - FH) / 4;
     const float* const u0 = a.in1 + gl * a.in1stride;
@@ -308,12 +308,12 @@ __global__ void __launch_bounds__(SW * 32, 4) k_stream_adj(DevGeo g, StreamAdj a
     const int y0 = id / a.strips % a.bands * a.R, yend = min(y0 + a.R, ny);
     // per warp: z1, z2, correlation, L_1 .. L_T [AD][AW]; c, d [AC][AW]; receivers and their residuals
     constexpr int WF = (AD * (3 + T) + 2 * AC) * AW;
-    float* const base = reinterpret_cast<float*>(smem4) + w * (WF + MAXR + 16 + 2 * NREC + T * NREC);
+    float* const base = reinterpret_cast<float*>(smem4) + w * (WF + MAXR + 16 + NREC + T * NREC);
     float* const rz = base + 2 * lane;                     // this lane's places
     constexpr int Y = 3 * AW, KK = 6 * AW, LL = 9 * AW, C = (9 + 3 * T) * AW, DD = AC * AW;
     RowRec* const rows = reinterpret_cast<RowRec*>(base + WF);
     int* const ent = reinterpret_cast<int*>(base + WF + MAXR + 16);
-    float* const val = base + WF + MAXR + 16 + 2 * NREC;   // [T][NREC]
+    float* const val = base + WF + MAXR + 16 + NREC;   // [T][NREC]
     if (gl >= a.ng) return;
     const bool own = i >= 0 && i < g.nx && lane >= 2 && lane <= 29;
     const float* const z1 = a.in1 + gl * a.instride;
@@ -507,8 +507,11 @@ __global__ void k_zero_frame(float* __restrict__ p, int nx, int ny, int px, int6
     for (int64_t q = head + (int64_t)(ny - 1) * px + nx + t; q < ns; q += n) d[q] = 0.f;
 }
 
-constexpr size_t fwd_smem() { return 4 * (size_t)SW * ((2 * FD + FC) * FW + 2 * MAXR + 16 + 2 * NREC); }
-constexpr size_t adj_smem(int T) { return 4 * (size_t)SW * ((AD * (3 + T) + 2 * AC) * AW + MAXR + 16 + 2 * NREC + T * NREC); }
+// Four blocks fit an SM's 228 KB with 1 KB each for the system (with three the gradient share of 8 groups of 2048 x
+// 2048 took 59.5 ms, not 56).
+constexpr size_t fwd_smem() { return 4 * (size_t)SW * ((2 * FD + FC) * FW + 2 * MAXR + 16 + NREC); }
+constexpr size_t adj_smem(int T) { return 4 * (size_t)SW * ((AD * (3 + T) + 2 * AC) * AW + MAXR + 16 + NREC + T * NREC); }
+static_assert(4 * (fwd_smem() + 1024) <= 228 * 1024 && 4 * (adj_smem(4) + 1024) <= 228 * 1024, "four blocks per SM");
 
 // Rows of a band.  A block's time grows with the R + 2 T rows it computes; four blocks are resident on an
 // SM, and an SM with fewer than about 2.5 waits on latency, so a last wave of one block per SM costs as much

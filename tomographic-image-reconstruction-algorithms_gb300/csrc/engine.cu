@@ -719,12 +719,24 @@ tomo_status make_plan(tomo_ctx* c) {
         return plan_of(c, false, std::max(2, (int)std::ceil(std::sqrt(2.0 * (double)(nt - 2)))));
     };
     Plan p = choose();
-    if (p.P < 1 && c->NS != g.N) {   // the padded slices do not fit: the per-step kernels' may
-        c->res = c->res1 = ResShape{};
-        c->res_cands.clear();
+    if (c->NS != g.N) {
+        // Where the padded slices do not fit, or the streamed sweeps' frame and ring (about a tenth more) cost
+        // another pass or the full history, the per-step kernels' plan is taken: 512 x 512, 5120 steps, 32 groups in
+        // 7.5 GB: 271 ms an iteration in one pass of the strip kernels, 405 in what is left to the streamed.
+        const int64_t padded = c->NS;
+        const bool streamed = c->stream_ok;
         c->stream_ok = false;
         c->NS = g.N;
-        p = choose();
+        const Plan q = choose();
+        auto passes = [&](const Plan& x) { return (G + x.P - 1) / x.P; };
+        if (q.P >= 1 && (p.P < 1 || (streamed && (passes(q) < passes(p) || (q.full && !p.full))))) {
+            c->res = c->res1 = ResShape{};
+            c->res_cands.clear();
+            p = q;
+        } else {
+            c->stream_ok = streamed;
+            c->NS = padded;
+        }
     }
     if (p.P < 1)
         return c->fail(TOMO_ERR_OOM, "plan needs %.2f GB for one group per pass, %.2f GB available",

@@ -296,6 +296,34 @@ TileAdj tile_adj_args(tomo_ctx* c, int kz0, int T, int g0, int ng) {
     return a;
 }
 
+// Adjoint steps timed outside a pass (kernel trials, tomo_time_kernel) add their products to a scratch
+// correlation: c->corr holds the results of earlier passes, which a trial between two passes of a gradient, or
+// between two calls, must leave alone.  The scratch is memory only a pass uses and no timed step touches: the
+// streamed sweeps' framed correlation, else the first two slices of each group's checkpoints, else, with the
+// full history, slot 0 of each group (timed steps read slices from 1 on).
+float* trial_corr(const tomo_ctx* c, int64_t* stride) {
+    if (c->corrp) {
+        *stride = c->NS;
+        return c->corrp;
+    }
+    if (!c->full) {
+        *stride = (int64_t)c->nchunk * 2 * c->NS;
+        return c->ckpt;
+    }
+    *stride = (int64_t)c->S * c->geo.N;
+    return c->hist;
+}
+AdjStep trial_adj_args(tomo_ctx* c, int q, int ng) {
+    AdjStep as = adj_args(c, q, 0, ng);
+    as.corr = trial_corr(c, &as.cstride);
+    return as;
+}
+TileAdj trial_tile_adj_args(tomo_ctx* c, int kz0, int T, int ng) {
+    TileAdj a = tile_adj_args(c, kz0, T, 0, ng);
+    a.corr = trial_corr(c, &a.cstride);
+    return a;
+}
+
 // Forward steps of the next tile launch when L remain: at most 8, and at most S - 2 so the
 // slices it writes never land on the two slots it reads.
 int tile_fwd_steps(const tomo_ctx* c, int L) { return std::min(std::min(L, TILE_MAX_FWD), c->S - 2); }
@@ -437,7 +465,7 @@ tomo_status autotune(tomo_ctx* c) {
                 CU(c, cudaEventRecord(c->ev0, c->st));
                 for (int t = 0; t < reps; ++t) {
                     if (which == 0) launch_fwd_strip(rows, c->dg, c->coef, fwd_args(c, k0 + t, 0, ng), c->st);
-                    else launch_adj_strip(rows, which - 1, c->dg, c->coef, adj_args(c, k0 + reps - t, 0, ng), c->st);
+                    else launch_adj_strip(rows, which - 1, c->dg, c->coef, trial_adj_args(c, k0 + reps - t, ng), c->st);
                 }
                 CU(c, cudaEventRecord(c->ev1, c->st));
                 CU(c, cudaEventSynchronize(c->ev1));
@@ -485,8 +513,8 @@ tomo_status autotune(tomo_ctx* c) {
             for (int pass = 0; pass < passes; ++pass) {
                 CU(c, cudaEventRecord(c->ev0, c->st));
                 for (int t = 0; t < reps; t += 2)
-                    launch_adj2_strip(code, c->dg, c->coef, adj_args(c, k0 + reps - t, 0, ng),
-                                      adj_args(c, k0 + reps - t - 1, 0, ng), c->st);
+                    launch_adj2_strip(code, c->dg, c->coef, trial_adj_args(c, k0 + reps - t, ng),
+                                      trial_adj_args(c, k0 + reps - t - 1, ng), c->st);
                 CU(c, cudaEventRecord(c->ev1, c->st));
                 CU(c, cudaEventSynchronize(c->ev1));
                 float t_ms = 0.f;
@@ -537,7 +565,7 @@ tomo_status autotune(tomo_ctx* c) {
                 if (pass > 0) tf = std::min(tf, t_ms);
                 CU(c, cudaEventRecord(c->ev0, c->st));
                 for (const int kz : {k0 + reps + 1, k0 + reps - 5}) {
-                    TileAdj aa = tile_adj_args(c, kz, kz == k0 + reps + 1 ? 6 : 2, 0, n);
+                    TileAdj aa = trial_tile_adj_args(c, kz, kz == k0 + reps + 1 ? 6 : 2, n);
                     aa.warps = warps;
                     launch_adj_tile(c->dg, c->tmaps, aa, c->st);
                 }
@@ -593,11 +621,11 @@ tomo_status autotune(tomo_ctx* c) {
                 CU(c, cudaEventRecord(c->ev0, c->st));
                 for (int t = 0; t < reps;) {
                     if (c->adj_pair) {
-                        launch_adj2_strip(c->rows_adj2, c->dg, c->coef, adj_args(c, k0 + reps - t, 0, 1),
-                                          adj_args(c, k0 + reps - t - 1, 0, 1), c->st);
+                        launch_adj2_strip(c->rows_adj2, c->dg, c->coef, trial_adj_args(c, k0 + reps - t, 1),
+                                          trial_adj_args(c, k0 + reps - t - 1, 1), c->st);
                         t += 2;
                     } else {
-                        launch_adj_strip(c->rows_adj, c->adj_variant, c->dg, c->coef, adj_args(c, k0 + reps - t, 0, 1),
+                        launch_adj_strip(c->rows_adj, c->adj_variant, c->dg, c->coef, trial_adj_args(c, k0 + reps - t, 1),
                                          c->st);
                         t += 1;
                     }
@@ -1517,7 +1545,7 @@ void enqueue_steps(tomo_ctx* c, int which, int k0, int steps, int ng, bool keep)
             t += T;
         } else if (which == 1 && (ng == 1 ? c->tile_adj1 : c->tile_adj)) {
             const int T = tile_adj_steps(steps - t);
-            launch_adj_tile(c->dg, c->tmaps, tile_adj_args(c, k0 + steps - t, T, 0, ng), c->st);
+            launch_adj_tile(c->dg, c->tmaps, trial_tile_adj_args(c, k0 + steps - t, T, ng), c->st);
             t += T;
         } else if (which == 0 && c->fwd_pair && t + 1 < steps) {
             launch_fwd2_strip(c->rows_fwd2, c->dg, c->coef, fwd_args(c, k0 + t, 0, ng), fwd_args(c, k0 + t + 1, 0, ng),
@@ -1528,10 +1556,10 @@ void enqueue_steps(tomo_ctx* c, int which, int k0, int steps, int ng, bool keep)
             t += 1;
         } else if (c->adj_pair && t + 1 < steps) {
             const int q = k0 + steps - 1 - t;
-            launch_adj2_strip(c->rows_adj2, c->dg, c->coef, adj_args(c, q, 0, ng), adj_args(c, q - 1, 0, ng), c->st);
+            launch_adj2_strip(c->rows_adj2, c->dg, c->coef, trial_adj_args(c, q, ng), trial_adj_args(c, q - 1, ng), c->st);
             t += 2;
         } else {
-            adj_launch(c, adj_args(c, k0 + steps - 1 - t, 0, ng));
+            adj_launch(c, trial_adj_args(c, k0 + steps - 1 - t, ng));
             t += 1;
         }
     }

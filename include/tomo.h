@@ -373,7 +373,9 @@ tomo_status tomo_iterate_batch(tomo_ctx** ctxs, int32_t n, int32_t method, const
  * as kernel arguments, so no device work refers to host memory after the call
  * returns.  All calls on a device share the one array: calls that overlap on
  * the GPU (concurrent streams or threads) race, so serialise them on one
- * stream. */
+ * stream.  Grids that fit on chip are solved by blocks that wait for each
+ * other, at most one second; where such a wait runs out (tomo_create's contexts
+ * report TOMO_ERR_TIMEOUT) every record of that group is NaN. */
 tomo_status tomo_forward_noalloc(const tomo_config* cfg, const float* d_f, float* d_records,
                                  void* stream);
 

@@ -347,6 +347,7 @@ struct ResFwd {
     int nwarps;
     float* out;                     // u(k0+T) in natural order (null: none)
     int64_t outstride;
+    bool nan_on_timeout;            // a group with a wait that ran out leaves NaN records (callers that cannot read w.err)
     TileWait w;
 };
 struct ResAdj {

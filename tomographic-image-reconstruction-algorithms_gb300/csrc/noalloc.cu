@@ -37,7 +37,8 @@
 //
 // All calls share the one array and it keeps the last call's contents: each
 // call zeroes the time slots it starts from and the output records,
-// and rewrites everything else before reading it.  Calls that overlap on the
+// and rewrites everything else before reading it.  The blocks of a cluster wait for each other's rows, at most
+// a second; the call has returned by then, so a group whose wait runs out leaves NaN in all its records.  Calls that overlap on the
 // GPU (concurrent streams, or threads, on the same device) race on the array:
 // serialise them on one stream.
 #include <cuda_runtime.h>
@@ -196,7 +197,7 @@ extern "C" tomo_status tomo_forward_noalloc(const tomo_config* cfg, const float*
     } else {
         dg.rcv = put(geo.rcv.data(), nch);
     }
-    // the word the kernels' bounded waits would set; nothing reads it
+    // the word the kernels' bounded waits set; the kernel itself reads it at its end (nan_on_timeout)
     static const uint32_t zero = 0;
     unsigned int* const err = (unsigned int*)put(&zero, 1);
     if ((s = put_words((uint32_t*)src, words.data(), (int64_t)words.size(), st)) != TOMO_OK) return s;
@@ -233,7 +234,10 @@ extern "C" tomo_status tomo_forward_noalloc(const tomo_config* cfg, const float*
         r.ng = geo.G;
         r.cs = shape.cs;
         r.gout = d_records;
-        r.w = TileWait{err, 1000000000ull, 0u, nullptr, 0u};
+        r.nan_on_timeout = true;
+        r.w = TileWait{err, 1000000000ull, 0u, nullptr, 0u};   // the contexts' bound, and their variables
+        if (const char* v = std::getenv("TOMO_WAIT_LIMIT_NS")) r.w.wait_ns = std::strtoull(v, nullptr, 10);
+        if (const char* v = std::getenv("TOMO_TEST_UNDELIVERED_TX")) r.w.extra_tx = (uint32_t)std::strtoul(v, nullptr, 10);
         launch_res_fwd(shape, dg, r, st);
         NA_CU(cudaGetLastError());
         return TOMO_OK;

@@ -416,6 +416,7 @@ __global__ void __launch_bounds__(MAXT, 1) k_ref_fwd(DevGeo g, ResFwd a) {
     }
     cp_async_wait<0>();
     cluster_sync();
+    res_timeout_records(g, a, gl, rank, cs);
 }
 
 // A row of quotients x / HH, HH = h^2: a product with the rounded reciprocal y, its exact remainder

@@ -46,7 +46,7 @@ DRIVERS = {
     "tomo": "TOMO_MULTI",
 }
 HEADERS = [os.path.join(INCLUDE, "tomo.h"), os.path.join(CSRC, "internal.h"), os.path.join(CSRC, "cell.cuh"),
-           os.path.join(CSRC, "async.cuh"), os.path.join(CSRC, "resident.cuh"), os.path.join(CSRC, "resident_ref.cuh"), os.path.join(CSRC, "cnn.h")]
+           os.path.join(CSRC, "async.cuh"), os.path.join(CSRC, "bounded_wait.h"), os.path.join(CSRC, "resident.cuh"), os.path.join(CSRC, "resident_ref.cuh"), os.path.join(CSRC, "cnn.h")]
 
 
 def _newer(target: str, deps: list[str]) -> bool:

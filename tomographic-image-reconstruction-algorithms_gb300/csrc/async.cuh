@@ -2,7 +2,7 @@
 // mbarriers with waits bounded by %globaltimer, TMA tile copies (cp.async.bulk.tensor) and the
 // fifth-generation tensor cores (tcgen05: TMEM allocation, MMA from shared-memory descriptors,
 // commit to an mbarrier, accumulator loads).  Included inside an anonymous namespace by the
-// translation units that use it (tile.cu, cnn.cu).
+// translation units that use it (tile.cu, cnn.cu, resident.cuh), after bounded_wait.h.
 //
 // Every wait here is bounded: a caller that sees a time-out records it in a host-visible error
 // word and leaves its kernel, so no copy or MMA that never completes can hang the GPU.
@@ -41,27 +41,17 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
 }
 // Waits for phase `parity` of the barrier to complete, at most limit_ns; false on time-out.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint64_t limit_ns) {
-    if (mbar_try_wait(bar, parity)) return true;
-    const uint64_t t0 = gtimer();
-    do {
-        if (mbar_try_wait(bar, parity)) return true;
-    } while (gtimer() - t0 < limit_ns);
-    return false;
+    return bounded_wait([&] { return mbar_try_wait(bar, parity); }, [] { return gtimer(); },
+                        [&](uint64_t t0) { return gtimer() - t0 < limit_ns; });
 }
 
 // Wait of one role of a warp-specialised kernel: gives up when the barrier has not completed
 // within limit_ns (raising the block's abort flag) or when another role has raised it.
 __device__ __forceinline__ bool role_wait(uint64_t* bar, uint32_t parity, uint64_t limit_ns, volatile int* abort) {
-    if (mbar_try_wait(bar, parity)) return true;
-    const uint64_t t0 = gtimer();
-    for (;;) {
-        if (mbar_try_wait(bar, parity)) return true;
-        if (*abort) return false;
-        if (gtimer() - t0 >= limit_ns) {
-            *abort = 1;
-            return false;
-        }
-    }
+    const bool ok = bounded_wait([&] { return mbar_try_wait(bar, parity); }, [] { return gtimer(); },
+                                 [&](uint64_t t0) { return !*abort && gtimer() - t0 < limit_ns; });
+    if (!ok) *abort = 1;
+    return ok;
 }
 
 // Device-scope acquire load (a spin on a counter other blocks release into).

@@ -44,6 +44,7 @@
 #include <cstdint>
 #include <cstring>
 
+#include "bounded_wait.h"
 #include "cnn.h"
 #include "internal.h"
 

@@ -40,6 +40,7 @@
 #include <cstdlib>
 #include <type_traits>
 
+#include "bounded_wait.h"
 #include "internal.h"
 
 namespace tomo {
@@ -86,12 +87,8 @@ __device__ __forceinline__ bool try_wait_cluster(uint32_t bar, uint32_t parity) 
 }
 // A warp's wait for a neighbour's row, at most limit_ns; the same answer in every lane.
 __device__ __forceinline__ bool wait_row(uint32_t bar, uint32_t parity, uint64_t limit_ns) {
-    if (__all_sync(FULL, try_wait_cluster(bar, parity))) return true;
-    const uint64_t t0 = gtimer();
-    do {
-        if (__all_sync(FULL, try_wait_cluster(bar, parity))) return true;
-    } while (__all_sync(FULL, gtimer() - t0 < limit_ns));
-    return false;
+    return bounded_wait([&] { return __all_sync(FULL, try_wait_cluster(bar, parity)) != 0; }, [] { return gtimer(); },
+                        [&](uint64_t t0) { return __all_sync(FULL, gtimer() - t0 < limit_ns) != 0; });
 }
 
 // Geometry of one instantiation.

@@ -39,6 +39,7 @@
 #include <cstring>
 #include <string>
 
+#include "bounded_wait.h"
 #include "internal.h"
 
 namespace tomo {
@@ -154,15 +155,9 @@ __device__ __forceinline__ bool grid_sync(const TileWait& w, unsigned int chunk)
         __threadfence();
         atomicAdd(w.gbar, 1u);
         const unsigned int target = gridDim.x * gridDim.y * chunk + w.gbar_extra;
-        if (ld_acquire(w.gbar) < target) {
-            const uint64_t t0 = gtimer();
-            while (ld_acquire(w.gbar) < target)
-                if (gtimer() - t0 >= w.wait_ns) {
-                    ok = false;
-                    atomicOr(w.err, 1u);
-                    break;
-                }
-        }
+        ok = bounded_wait([&] { return ld_acquire(w.gbar) >= target; }, [] { return gtimer(); },
+                          [&](uint64_t t0) { return gtimer() - t0 < w.wait_ns; });
+        if (!ok) atomicOr(w.err, 1u);
         fence_proxy_async_global();   // this thread's next TMA copies see the other blocks' writes
     }
     return __syncthreads_and(ok);

@@ -197,7 +197,7 @@ extern "C" tomo_status tomo_forward_noalloc(const tomo_config* cfg, const float*
     } else {
         dg.rcv = put(geo.rcv.data(), nch);
     }
-    // the word the kernels' bounded waits set; the kernel itself reads it at its end (nan_on_timeout)
+    // the word the kernels' bounded waits set; the caller learns of them by the records (nan_on_timeout)
     static const uint32_t zero = 0;
     unsigned int* const err = (unsigned int*)put(&zero, 1);
     if ((s = put_words((uint32_t*)src, words.data(), (int64_t)words.size(), st)) != TOMO_OK) return s;

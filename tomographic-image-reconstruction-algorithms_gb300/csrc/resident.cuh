@@ -343,14 +343,15 @@ __device__ __forceinline__ void res_checkpoint(const ResFwd& a, int gl, int64_t 
     }
 }
 
-// The records of a group for a caller that cannot be told of a wait that ran out: all NaN.  Called by every
-// block after the cluster's last barrier, behind which the notes and the records of all its blocks are (a
-// block can finish on rows computed past a neighbour's failed wait, so the whole group is given up).  One warp
-// looks: with every thread of 128 blocks loading the same word, 128 x 128 and 600 steps took 3 us longer.
-__device__ __forceinline__ void res_timeout_records(const DevGeo& g, const ResFwd& a, int gl, int rank, int cs) {
-    if (!a.nan_on_timeout || threadIdx.x >= 32 || ld_acquire(a.w.err) == 0u) return;
-    const int64_t n = (int64_t)g.nt * g.nch;
-    for (int64_t i = 32 * rank + threadIdx.x; i < n; i += 32 * cs) a.gout[gl * n + i] = __int_as_float(0x7fffffff);
+// The records of a group for a caller that cannot be told of a wait that ran out: all NaN.  Called by each block
+// with such a wait, behind the cluster's last barrier and so after every block's records (a block can finish on
+// rows computed past a neighbour's failed wait: the whole group is given up).  It stands in the failed branch and
+// reads the group's number again: behind the common path it cost the steps of one row per warp 2 to 5 %
+// (256 x 256, one group at a time: 59.9 -> 62.8 ms an iteration; as a launch of its own 5 us a call).
+__device__ __forceinline__ void res_nan_records(float* gout, int64_t n) {
+    uint32_t gl;
+    asm volatile("mov.u32 %0, %%clusterid.x;\n" : "=r"(gl));
+    for (int64_t i = threadIdx.x; i < n; i += blockDim.x) gout[gl * n + i] = __int_as_float(0x7fffffff);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -583,12 +584,17 @@ __global__ void __launch_bounds__(MAXT, 1) k_res_fwd(DevGeo g, ResFwd a) {
                     else F::store_nat(o, ua[r], lane, nx);
                 }
         }
-    } else if (threadIdx.x == 0) {
-        atomicOr(a.w.err, 1u);
+    } else {
+        if (threadIdx.x == 0) atomicOr(a.w.err, 1u);
+        if (a.nan_on_timeout) {
+            cp_async_wait<0>();
+            cluster_sync();
+            res_nan_records(a.gout, (int64_t)g.nt * g.nch);
+            return;
+        }
     }
     cp_async_wait<0>();
     cluster_sync();            // no block leaves while another may still write its shared memory
-    res_timeout_records(g, a, gl, rank, cs);
 }
 
 // ---------------------------------------------------------------------------------------------

@@ -411,12 +411,17 @@ __global__ void __launch_bounds__(MAXT, 1) k_ref_fwd(DevGeo g, ResFwd a) {
                     else F::store_nat(o, ua[r], lane, nx);
                 }
         }
-    } else if (threadIdx.x == 0) {
-        atomicOr(a.w.err, 1u);
+    } else {
+        if (threadIdx.x == 0) atomicOr(a.w.err, 1u);
+        if (a.nan_on_timeout) {
+            cp_async_wait<0>();
+            cluster_sync();
+            res_nan_records(a.gout, (int64_t)g.nt * g.nch);
+            return;
+        }
     }
     cp_async_wait<0>();
     cluster_sync();
-    res_timeout_records(g, a, gl, rank, cs);
 }
 
 // A row of quotients x / HH, HH = h^2: a product with the rounded reciprocal y, its exact remainder

@@ -2,8 +2,8 @@
 
 Kernels are chosen when a pass of one group, or of several, first runs, which can be in the middle of a
 gradient (a last pass of one group) or between two calls whose correlations stay in the context (group
-ranges of unequal lengths).  The first results of a fresh context must equal its second ones, and those of
-a context that keeps to the per-step kernels, bit for bit.  Grids: too large to stay on chip, a width that
+ranges of unequal lengths).  Trials also write residual records, which a pass must find as if there had been none.  The first results of a fresh context must equal its second ones, and those of
+a context that keeps to the per-step kernels, bit for bit.  Grids: one that stays on chip; too large for it, a width that
 is a multiple of four and enough steps for the trials; passes of several groups below and above the 32 MiB
 from which they are streamed without a trial (above it, the per-step kernels' own trials come with the
 first pass of one group, and run on as many groups as a pass holds).
@@ -32,6 +32,7 @@ CASES = {
     "passes of 4, 4 and 1": SMALL,
     "checkpoints": ring(448, 9, 4, 15),
     "timed memory plan": ring(448, 9, 4, -1),
+    "held on chip": ring(128, 9, 4, 15),
     "above 32 MiB a slice": ring(1024, 9, 8, 12),
     "above 32 MiB a slice, full history": ring(1024, 9, 8, 0),
 }
@@ -60,6 +61,7 @@ def test_first_gradient_equals_the_second(name, monkeypatch):
     assert np.array_equal(d1, d2) and r1 == r2
     assert all(np.abs(g).max() > 0 for g in first)
     monkeypatch.setenv("TOMO_STREAM", "0")
+    monkeypatch.setenv("TOMO_RESIDENT", "0")
     with tomo.Context(cfg) as ctx:
         want, d, r = ctx.gradient(f0, rec)
     assert np.array_equal(first, want) and np.array_equal(d1, d) and r1 == r

@@ -1476,13 +1476,18 @@ tomo_status tune_resident(tomo_ctx* c, int groups) {
     const bool tlog = std::getenv("TOMO_TUNE_LOG") != nullptr;
     // long enough that a launch's set-up does not decide, where a step is short
     const int T = std::min(std::min(c->K, g.nt - 2), (double)ng * g.N < 1e6 ? 96 : (double)ng * g.N < 2e6 ? 32 : 16);
+    // forward steps with records from the first slice without a source: nearly all steps of a sweep are such, and
+    // those with a source order the shapes otherwise (one group of 256 x 256: 1 and 2 rows per warp 102 and 93 us per
+    // 72 steps, 61 and 55 ms an iteration; with a source 100 and 99, so that chance chose between 61 and 55)
+    const int k0 = std::max(1, std::min(g.n_src_steps, g.nt - 1 - T));
     float best = 1e30f;
     for (const ResShape& s : cands) {
         float ms = 1e30f;
         for (int pass = 0; pass < 3; ++pass) {   // the first warms up
-            ResFwd f = res_fwd_args(c, s, 1, T, 0, ng);
+            ResFwd f = res_fwd_args(c, s, k0, T, 0, ng);
             f.hist = c->hist;
-            f.qlo = 1;
+            f.qlo = k0;
+            f.gout = c->rr;
             ResAdj a = res_adj_args(c, s, g.ref ? T : T + 1, T, 0, ng);
             a.qlo = 1;
             a.first = true;

@@ -670,15 +670,19 @@ double plan_bytes_per_group(const tomo_ctx* c, bool full, int K) {
     return 4.0 * ((double)(slots + tomo_ctx::ZR + 2 * chunks + more) * c->NS + (double)nt * g.nch);
 }
 
-// The plan with the most groups per pass that fits c->plan_budget (or the configured P).
+// Bytes the buffers of all groups of a pass may take together: the streamed sweeps hold a framed coefficient and
+// sponge map beside them.
+double plan_room(const tomo_ctx* c) { return c->plan_budget - (c->stream_ok ? 8.0 * (double)c->NS : 0.0); }
+
+// The plan with the most groups per pass that fits plan_room (or the configured P).
 Plan plan_of(const tomo_ctx* c, bool full, int K) {
     const Geometry& g = c->geo;
     Plan p{full, full ? g.nt - 2 : K, 0};
     const double per = plan_bytes_per_group(c, full, K);
     int P = g.cfg.groups_per_pass > 0 ? std::min(g.cfg.groups_per_pass, g.G) : g.G;
     if (g.cfg.groups_per_pass <= 0)
-        while (P > 1 && per * P > c->plan_budget) --P;
-    p.P = per * P <= c->plan_budget ? P : 0;
+        while (P > 1 && per * P > plan_room(c)) --P;
+    p.P = per * P <= plan_room(c) ? P : 0;
     return p;
 }
 
@@ -768,7 +772,7 @@ tomo_status make_plan(tomo_ctx* c) {
     }
     if (p.P < 1)
         return c->fail(TOMO_ERR_OOM, "plan needs %.2f GB for one group per pass, %.2f GB available",
-                       plan_bytes_per_group(c, p.full, p.K) / 1e9, c->plan_budget / 1e9);
+                       plan_bytes_per_group(c, p.full, p.K) / 1e9, plan_room(c) / 1e9);
     set_plan(c, p);
     return TOMO_OK;
 }

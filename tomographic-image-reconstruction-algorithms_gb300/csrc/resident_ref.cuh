@@ -431,8 +431,8 @@ __global__ void __launch_bounds__(MAXT, 1) k_ref_fwd(DevGeo g, ResFwd a) {
 // magnitude down to the smallest subnormal, so the row is scaled by 2^64 first and back afterwards,
 // which is exact but for quotients that are subnormal themselves, of x = 1 .. 8 x 2^-149; there the
 // second rounding goes wrong for 5 and 6, by one unit, which is taken back.  Tested against division
-// for every significand and in the subnormal range.  A lane with a value above 2^60 divides.  (A zero
-// keeps only its value, not its sign.)
+// for every significand and in the subnormal range.  The scaled quotient is x 2^64 10^6, below 2^127 up
+// to x = 2^43; a lane with a value above that divides.  (A zero keeps only its value, not its sign.)
 __device__ __forceinline__ float tiny_quotient(float q, float x) {
     const uint32_t b = 2u * __float_as_uint(x);
     return b == 10u || b == 12u ? __uint_as_float(__float_as_uint(q) - 1u) : q;
@@ -447,7 +447,7 @@ __device__ __forceinline__ void div_hh(float2 (&x)[NP]) {
         most = fmaxf(most, fmaxf(fabsf(x[v].x), fabsf(x[v].y)));
         least = min(least, min(2u * __float_as_uint(x[v].x) - 1u, 2u * __float_as_uint(x[v].y) - 1u));
     }
-    if (most > 0x1p60f) {
+    if (most > 0x1p43f) {
 #pragma unroll
         for (int v = 0; v < NP; ++v) x[v] = make_float2(__fdiv_rn(x[v].x, HH), __fdiv_rn(x[v].y, HH));
         return;

@@ -47,3 +47,15 @@ def test_row_that_never_arrives_leaves_nan(built_lib, name, monkeypatch):
     with tomo.Context(cfg) as ctx:
         want = ctx.forward(fo)
     assert np.array_equal(got, want) and np.abs(want).max() > 0
+
+
+def test_context_names_the_row(built_lib, monkeypatch):
+    """The contexts' message covers both kinds of wait: a resident sweep has no TMA copy."""
+    cfg = CASES["ring"]()
+    monkeypatch.setenv("TOMO_WAIT_LIMIT_NS", "2000000")
+    monkeypatch.setenv("TOMO_TEST_UNDELIVERED_TX", "16")
+    monkeypatch.setenv("TOMO_RES_SHAPE", "16,1")
+    with tomo.Context(cfg) as ctx:
+        with pytest.raises(tomo.TomoError) as e:
+            ctx.forward(np.zeros((cfg.ny, cfg.nx), np.float32))
+    assert e.value.status == tomo.ERR_TIMEOUT and "row did not arrive" in str(e.value), e.value

@@ -107,9 +107,9 @@ struct tomo_ctx {
     static constexpr int UR = STREAM_RING; // wavefield ring slots of the streamed sweeps
     TileMaps tmaps;              // TMA maps of hist, z, coef, dmap, rid (tile kernels)
     TileMaps tmaps_ck;           // the same with the slice maps over the checkpoint buffer (pass_layout)
-    unsigned int* err_host = nullptr;   // tile kernels' wait time-out word (mapped pinned memory)
+    unsigned int* err_host = nullptr;   // the kernels' wait time-out word (mapped pinned memory)
     unsigned int* err_dev = nullptr;
-    uint64_t wait_ns = 1000000000ull;   // bound of every tile-kernel copy wait (TOMO_WAIT_LIMIT_NS)
+    uint64_t wait_ns = 1000000000ull;   // bound of every wait in a kernel (TOMO_WAIT_LIMIT_NS)
     uint32_t test_tx = 0;        // TOMO_TEST_UNDELIVERED_TX: bytes a region barrier expects in vain
     unsigned int* gbar = nullptr;  // grid barrier counter of the persistent tile launches
     uint32_t test_gbar = 0;      // TOMO_TEST_GRID_BARRIER_EXTRA: arrivals a grid barrier waits for in vain
@@ -347,12 +347,12 @@ void encode_maps(tomo_ctx* c) {
                          (int64_t)c->P * tomo_ctx::ZR, c->coef, nullptr);
 }
 
-// Stream synchronisation that also reports a tile kernel's timed-out copy wait.
+// Stream synchronisation that also reports a timed-out wait (a tile kernel's copy, a resident sweep's row).
 tomo_status sync_check(tomo_ctx* c) {
     CU(c, cudaStreamSynchronize(c->st));
     if (c->err_host && *(volatile unsigned int*)c->err_host) {
         *(volatile unsigned int*)c->err_host = 0u;
-        return c->fail(TOMO_ERR_TIMEOUT, "tile kernel: a TMA copy did not arrive within %llu ns",
+        return c->fail(TOMO_ERR_TIMEOUT, "a TMA copy or a neighbouring block's row did not arrive within %llu ns",
                        (unsigned long long)c->wait_ns);
     }
     return TOMO_OK;
@@ -890,7 +890,7 @@ tomo_status create_buffers(tomo_ctx* c) {
         launch_frame(c->dmapp, c->dmap, g.nx, g.ny, c->st);
     }
     c->strip = strip_supported(d, g.cfg.profile) && !std::getenv("TOMO_NO_STRIP");
-    // the tile kernels' wait time-out word, written by the device, read by sync_check
+    // the kernels' wait time-out word, written by the device, read by sync_check
     // (and, 64 bytes on, the results a call reads back: pin)
     CU(c, cudaHostAlloc((void**)&c->err_host, 128, cudaHostAllocMapped));
     *c->err_host = 0u;
@@ -2094,7 +2094,7 @@ tomo_status iterate_batch_graph(tomo_ctx** ctxs, int n, int method, const tomo_s
             tomo_ctx* c = ctxs[i];
             if (c->err_host && *(volatile unsigned int*)c->err_host) {
                 *(volatile unsigned int*)c->err_host = 0u;
-                return c->fail(TOMO_ERR_TIMEOUT, "tile kernel: a TMA copy did not arrive within %llu ns",
+                return c->fail(TOMO_ERR_TIMEOUT, "a TMA copy or a neighbouring block's row did not arrive within %llu ns",
                                (unsigned long long)c->wait_ns);
             }
             c->launches += lead->batch_kernels[i];

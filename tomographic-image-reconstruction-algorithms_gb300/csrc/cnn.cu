@@ -95,10 +95,12 @@ struct ConvShape {
 // operand the weights of dy = 2, 1, 0, and the 3 N columns the neighbouring accumulators of the output rows
 // j - 2, j - 1, j), warps 2-5 drain the accumulators (their TMEM lane quarters are warp % 4) and store.
 // A row takes 7 or 8 MMAs of up to 96 columns where one per tap and 16 channels takes 18 of 32, and its slot is
-// free after them, not two rows later; 32 -> 32 channels, 512 x 512: 27.0 -> 24.5 us cold, 1 M pixels 40.9 -> 38
-// (the bytes take 20; at about 1300 multiply-adds per cycle and SM the tensor core is what the rows wait
-// for).  An accumulator's products come in the order (dy, dx, channels), as one MMA per tap gives them: same bits.  Barriers: full / empty per row slot (TMA transaction bytes /
-// MMA commit), full / empty per accumulator (MMA commit of its last input row / one arrival per epilogue warp).
+// free after them, not two rows later; 32 -> 32 channels under ncu: 512 x 512 15.5 -> 14.6 us, 1 M pixels
+// 39.8 -> 36.5.  What bounds a launch, from these two sizes: about 7 us whatever the size (set-up, weights, first
+// rows, last stores) and 7.3 us per 262144 pixels, in which their 33.5 MB go by at 4.6 TB/s; the tensor pipe is active
+// 16 and 24 % of the cycles.  An accumulator's products come in the order (dy, dx, channels), as one MMA per
+// tap gives them: same bits.  Barriers: full / empty per row slot (TMA transaction bytes / MMA commit), full /
+// empty per accumulator (MMA commit of its last input row / one arrival per epilogue warp).
 template <int CIN, int N, int EPI>
 __global__ void __launch_bounds__(192, 2) k_conv_tc(const __grid_constant__ CUtensorMap line_map, const __grid_constant__ CUtensorMap halo_map,
                                                     ConvArgs a, int RC) {
@@ -307,7 +309,7 @@ struct WgradArgs {
 // of 128 x 96 takes all nine taps in 8 MMAs per row.  With the copies on the input's side, three groups of (tap,
 // ci) rows and N = 32, it was 24 per row, and the copies of the wider operand left room for 5 input and 2
 // gradient rows in flight instead of 8 and 4.  Measured, 32 -> 32 channels,
-// 1 M pixels: 77 -> 42 us; the two operands' bytes take 20.
+// 1 M pixels: 77 -> 42 us; the two operands' bytes take 20, the tensor pipe is active 31 % of the cycles.
 template <int CIN, int NB>
 struct WgradShape {
     static constexpr int NCHX = CIN / 8;

@@ -1576,7 +1576,7 @@ void enqueue_steps(tomo_ctx* c, int which, int k0, int steps, int ng, bool keep)
 
 // Chooses between the streamed sweeps and the per-step (or tile) kernels autotune picks, for passes of one
 // group or of more (up to P).  Streamed without a trial: passes whose slices of all groups are a quarter of the
-// L2 or more, which are bound by bytes (iterations at 512 x 512, 32 groups: 134 -> 120 ms, 2048 x 2048, 8: 77 ->
+// GB300's 129 MB L2 or more, which are bound by bytes (iterations at 512 x 512, 32 groups: 134 -> 120 ms, 2048 x 2048, 8: 77 ->
 // 56; the trials and autotune's took 170 ms of a context's first pass), and widths that are not a multiple of 4,
 // which only the per-cell kernels take otherwise (403 x 390, 8 groups: 7.0 -> 3.8 ms together, 21.4 -> 17.4 one by
 // one).  Else steps of each are timed: a step of a pass costs a forward step with records, for all chunks but
@@ -1640,7 +1640,8 @@ tomo_status tune_stream(tomo_ctx* c, int groups) {
     TRY(time_steps(0, false, fn));
     TRY(time_steps(0, true, fk));
     TRY(time_steps(1, true, b));
-    pick = again * fn + fk + b < 0.92 * (f * (1.0 + again) + a);   // the steps with sources gain less
+    // 0.92: a margin for what the trial does not time, steps with sources and the pass's other launches
+    pick = again * fn + fk + b < 0.92 * (f * (1.0 + again) + a);
     if (std::getenv("TOMO_TUNE_LOG"))
         std::fprintf(stderr, "tomo tune: %d groups, us per step: per-step kernels forward %.2f adjoint %.2f, streamed forward "
                      "%.2f (with history %.2f) adjoint %.2f\n", ng, 1e3 * f / steps, 1e3 * a / steps, 1e3 * fn / steps,

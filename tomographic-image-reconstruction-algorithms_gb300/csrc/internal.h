@@ -375,7 +375,7 @@ struct ResAdj {
 int res_held(const ResShape& s);
 std::vector<ResShape> res_shapes(int nx, int ny, const std::vector<int32_t>& rowstart);
 // A shape for ng groups without timing the candidates: as many blocks per group as give every group its
-// own blocks on about 144 SMs, else the fewest; of equal ones the first listed (fewest rows per warp).
+// own blocks on about 144 of the GB300's 152 SMs (clusters of 16 leave some of the others idle), else the fewest; of equal ones the first listed (fewest rows per warp).
 ResShape res_pick(const std::vector<ResShape>& shapes, int ng);
 int64_t res_slice(const ResShape& s, int ny);   // floats of a slice in fragment order
 // Reference profile: the rows of each warp (first row, count in the high half; empty: not resident), and

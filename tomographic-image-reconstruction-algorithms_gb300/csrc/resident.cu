@@ -21,7 +21,11 @@ constexpr int kMaxCluster = 16;
 // Cells per lane of a grid width (0: too wide).  Shapes are limited by registers: the adjoint keeps
 // z, the previous z, its products and the correlation, 4 x cells per thread, beside about 90 others,
 // so a block of up to 8 warps (255 registers) takes 32 cells per thread and one of up to 16 warps
-// (128 registers) 16.  A 512 x 512 grid would need 64 cells per thread on 16 blocks: tried, it
+// (128 registers) 16.  The builds of up to 16 warps with the most cells spill (-Xptxas -v, bytes stored / loaded:
+// reference forward 10 cells per lane 512 / 784, 8 cells 196 / 288, adjoint 172 / 312 and 60 / 64; CFG adjoint 2 rows of
+// 8, 4 of 4 and 1 of 16 cells 110 to 130 / 160 to 190).  A context times its shapes, so they run only where they are
+// the faster ones; the allocation-free forward takes its shape untimed, and for reference grids of 288 rows has no
+// other.  A 512 x 512 grid would need 64 cells per thread on 16 blocks: tried, it
 // spills (41 us per adjoint step of 32 groups against 26 us in the strip kernels and 22 streamed), so such
 // grids are streamed or stay with the strip and tile kernels.
 int cells_per_lane(int nx) {

@@ -21,12 +21,14 @@
 // the width or alignment of the grid.
 //
 // Measured (one GB300, against the strip and tile kernels on the same grids): 128 x 128, 8 groups:
-// 0.33 / 0.38 us per forward / adjoint step (0.83 / 1.18), an iteration of 600 steps 0.60 ms (1.43);
+// 0.35 / 0.40 us per forward / adjoint step (0.83 / 1.18), an iteration of 600 steps 0.58 ms (1.43);
 // 256 x 256, one group: 0.42 / 0.62 us (1.2 / 1.6 us in multi-step tiles), an ART iteration of 16
-// groups x 2560 steps 58.7 ms (115.4); 301 x 233, 10 groups (per-cell kernels before): 1.3 / 1.6 us
-// (4.2 / 5.6), 3.06 ms per iteration (13.2).  What bounds a step: on small bands the step's
-// dependent chain (about 75 instructions at 7 cycles each), on large ones issue slots at two warps
-// per scheduler.
+// groups x 2560 steps 55 ms (115.4); 301 x 233, 10 groups (per-cell kernels before): 1.3 / 1.6 us
+// (4.2 / 5.6), 2.98 ms per iteration (13.2).  What bounds a step is latency.  ncu, forward sweeps with records:
+// 128 x 128, 8 groups on 12 blocks of 11 warps: 91 instructions per warp and step, 2.75 warps per scheduler, 32 %
+// of the cycles issue, the block barrier and fixed latencies the largest stalls (2.4 and 1.6 cycles per issue);
+// 256 x 256, one group on 16 blocks of 8 warps: 161 instructions, 2 warps per scheduler, 34 % (barrier 1.2, fixed
+// latencies 1.2).  DRAM is at 2 to 14 % of its peak.
 //
 // Waits: only the edge warps wait on other blocks, bounded by TileWait::wait_ns of %globaltimer; a
 // wait that runs out sets bit 0 of the host-visible error word and makes the cluster leave.

@@ -17,8 +17,9 @@
 // adjoint step (per-cell kernels: 13 us with the gather, 22), an iteration 5.6 ms (14.0); one group
 // of it on a cluster of 14 blocks 0.93 / 1.07 us (9.3 us for the three launches of a step before),
 // a sequential iteration of 32 groups 27.0 ms (119.6); data generation 2.2 ms (5.2).  What bounds a
-// step: the instruction stream of a warp's two rows (320 forward, 395 adjoint) at two to four warps per
-// scheduler, 30 to 45 % issue active.
+// step: the instruction stream of a warp's two rows.  ncu, one group of 192 x 192 on 14 blocks of 7 warps:
+// 327 instructions per warp and step forward, 421 adjoint, at 1.75 warps per scheduler; 29 and 33 % of the cycles
+// issue, fixed latencies (1.2 and 1.5 cycles per issue) and forward the block barrier (1.1) the largest stalls.
 #pragma once
 #include "resident.cuh"
 

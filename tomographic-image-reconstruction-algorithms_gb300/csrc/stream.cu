@@ -513,7 +513,7 @@ constexpr size_t fwd_smem() { return 4 * (size_t)SW * ((2 * FD + FC) * FW + 2 * 
 constexpr size_t adj_smem(int T) { return 4 * (size_t)SW * ((AD * (3 + T) + 2 * AC) * AW + MAXR + 16 + NREC + T * NREC); }
 static_assert(4 * (fwd_smem() + 1024) <= 228 * 1024 && 4 * (adj_smem(4) + 1024) <= 228 * 1024, "four blocks per SM");
 
-// Rows of a band.  A block's time grows with the R + 2 T rows it computes; four blocks are resident on an
+// Rows of a band (152: the SMs of a GB300).  A block's time grows with the R + 2 T rows it computes; four blocks are resident on an
 // SM, and an SM with fewer than about 2.5 waits on latency, so a last wave of one block per SM costs as much
 // as one of 2.5.  Measured forward us per step (without history), 32 groups of 512 x 512: R 28, 36, 64, 76,
 // 104: 11.0, 8.9, 11.4, 11.4, 15.4; 8 groups of 2048 x 2048: 29.4, 28.7, 27.2, 28.0, 32.8.  Adjoint: 24.7,
